@@ -13,32 +13,34 @@
 
 namespace ar
 {
-// Per-ray constants of the shear transform.
+// Per-ray constants of the shear transform.  kz is the direction's largest
+// axis; the other two follow in cyclic order.  The published method exchanges
+// them when the direction is negative along kz, which only negates the three
+// edge functions, their sum and T together (each is a difference or a sum of
+// the same rounded products), so every sign test and T / det come out the same
+// without the exchange.
 struct RayShear
 {
-    int kx, ky, kz;
+    int kz;
     float sx, sy, sz;
 };
+
+// (v[kz + 1], v[kz + 2], v[kz]), indices modulo 3
+AR_HD V3 shear_order(V3 v, int kz)
+{
+    return v3(kz == 0 ? v.y : (kz == 1 ? v.z : v.x), kz == 0 ? v.z : (kz == 1 ? v.x : v.y),
+              kz == 0 ? v.x : (kz == 1 ? v.y : v.z));
+}
 
 AR_HD RayShear make_shear(V3 d)
 {
     RayShear s;
     const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
     s.kz = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
-    s.kx = s.kz + 1;
-    if (s.kx == 3) s.kx = 0;
-    s.ky = s.kx + 1;
-    if (s.ky == 3) s.ky = 0;
-    if (comp(d, s.kz) < 0.0f)
-    {
-        const int t = s.kx;
-        s.kx = s.ky;
-        s.ky = t;
-    }
-    const float dz = comp(d, s.kz);
-    s.sx = comp(d, s.kx) / dz;
-    s.sy = comp(d, s.ky) / dz;
-    s.sz = 1.0f / dz;
+    const V3 p = shear_order(d, s.kz);
+    s.sx = p.x / p.z;
+    s.sy = p.y / p.z;
+    s.sz = 1.0f / p.z;
     return s;
 }
 
@@ -47,16 +49,16 @@ AR_HD RayShear make_shear(V3 d)
 AR_HD bool tri_intersect(const RayShear& s, V3 o, V3 v0, V3 v1, V3 v2,
                          float* t_out, float* b0_out, float* b1_out, float* b2_out)
 {
-    const V3 A = v0 - o;
-    const V3 B = v1 - o;
-    const V3 C = v2 - o;
-    const float Akz = comp(A, s.kz), Bkz = comp(B, s.kz), Ckz = comp(C, s.kz);
-    const float Ax = comp(A, s.kx) - s.sx * Akz;
-    const float Ay = comp(A, s.ky) - s.sy * Akz;
-    const float Bx = comp(B, s.kx) - s.sx * Bkz;
-    const float By = comp(B, s.ky) - s.sy * Bkz;
-    const float Cx = comp(C, s.kx) - s.sx * Ckz;
-    const float Cy = comp(C, s.ky) - s.sy * Ckz;
+    const V3 A = shear_order(v0 - o, s.kz);
+    const V3 B = shear_order(v1 - o, s.kz);
+    const V3 C = shear_order(v2 - o, s.kz);
+    const float Akz = A.z, Bkz = B.z, Ckz = C.z;
+    const float Ax = A.x - s.sx * Akz;
+    const float Ay = A.y - s.sy * Akz;
+    const float Bx = B.x - s.sx * Bkz;
+    const float By = B.y - s.sy * Bkz;
+    const float Cx = C.x - s.sx * Ckz;
+    const float Cy = C.y - s.sy * Ckz;
     float U = Cx * By - Cy * Bx;
     float V = Ax * Cy - Ay * Cx;
     float W = Bx * Ay - By * Ax;

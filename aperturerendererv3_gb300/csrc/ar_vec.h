@@ -51,7 +51,6 @@ AR_HD float max3(V3 a) { return fmaxf(a.x, fmaxf(a.y, a.z)); }
 AR_HD float sum3(V3 a) { return a.x + a.y + a.z; }
 AR_HD bool all_zero(V3 a) { return a.x == 0.0f && a.y == 0.0f && a.z == 0.0f; }
 AR_HD V3 reflect(V3 v, V3 n) { return v - 2.0f * dot(v, n) * n; }
-AR_HD float comp(V3 a, int k) { return k == 0 ? a.x : (k == 1 ? a.y : a.z); }
 AR_HD float lerpf(float a, float b, float t) { return a * (1.0f - t) + b * t; }
 AR_HD float signf(float a) { return a > 0.0f ? 1.0f : (a < 0.0f ? -1.0f : 0.0f); }
 AR_HD bool is_nanf(float x) { return x != x; }
