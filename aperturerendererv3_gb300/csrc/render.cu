@@ -724,6 +724,18 @@ __global__ void __launch_bounds__(AR_BLOCK) k_partition(const int* __restrict__ 
 #define AR_FEAT_ALL (AR_MATS_ALL | AR_FEAT_MEDIUM | AR_FEAT_TEX)
 #define AR_FEAT_SURFACE (AR_MATS_DIFFUSE | AR_MATS_LIGHT | AR_MATS_GGX)
 
+// What bounds k_shade is instruction supply: one vertex runs some 2,800
+// instructions of mostly straight-line code (45 KB), the SM holds 16 warps
+// (128 registers), and when each warp is somewhere else in that code most
+// stalls are instruction fetches (256x256x16 Cornell box: 3.7 of 10.4 warps per
+// issue; voxel guide: 14.0 of 21.5).  A barrier at the top of each pass and one
+// before next-event estimation keep a block's warps in the same part of the
+// code, so that a fetch serves all of them.  Measured, shading: 256x256x16
+// Cornell box 0.98 -> 0.90 ms, textured forward and backward step 27.3 -> 25.3 ms,
+// voxel guide 480x270x16 6.23 -> 4.29 ms.  The opaque-surface instantiation
+// keeps only the first one: its waves on large scenes wait for memory
+// (1920x1080x32 terrain 9.83 ms with one barrier, 10.04 with both, 9.89 with
+// none).  More barriers, or blocks of 512, gain nothing further.
 template <int GUIDE, bool ADJ, int FEAT = AR_FEAT_ALL>
 __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
                                             : (FEAT == AR_FEAT_SURFACE ? AR_SHADE_LEAN_MIN_BLOCKS : AR_SHADE_MIN_BLOCKS))
@@ -746,8 +758,10 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
     // read nothing of an ended path but its radiance.
     constexpr bool TRACK_MEDIA = (FEAT & AR_MATS_GLASS) != 0;
     constexpr bool STORE_ENDED = GUIDE != 0 || ADJ;
+    constexpr bool SYNC_NEE = FEAT != AR_FEAT_SURFACE;
     for (int bbase = blockIdx.x * blockDim.x; bbase < n; bbase += stride)
     {
+        __syncthreads();  // the block's warps start the pass together
         const int qq = bbase + (int)threadIdx.x;
         const bool active = qq < n;
         // the entry this thread shades in its next pass, read now; its state is
@@ -760,20 +774,43 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
         V3 sh_o = v3(0, 0, 0), sh_d = v3(0, 0, 0);
         float sh_tmax = 0.0f, sh_vun = 0.0f, sh_vocc = 0.0f, sh_sdf_eps = 0.0f;
         bool sh_valid = false;
+        // state of the vertex, across the phases below
+        V3 rayO = v3(0, 0, 0), rayD = v3(0, 0, 0);
+        float lambda = 0.0f, lambda_pdf = 0.0f, d65 = 0.0f, radiance = 0.0f, mask = 0.0f, eps = 0.0f;
+        Basis lb = {{0.0f, 0.0f, 0.0f, 0.0f}};
+        int depth = 0, ndd = 0, slot = -1, texel = -1;
+        uint32_t fl = 0u;
+        bool prev_did_nee = false, scatter = false, ended = true;
+        Media media = media_default();
+        DevRand R;
+        R.g.state = 0u;
+        R.g.inc = 0u;
+        Hit h;
+        h.hit = false;
+        h.obj = -1;
+        h.light = -1;
+        h.dist = 0.0f;
+        h.pos = v3(0, 0, 0);
+        h.nrm = v3(0, 0, 0);
+        h.local_pos = v3(0, 0, 0);
+        BsdfSample S = bsdf_sample_default();
+        Material mat;
+        mat.shading = AR_MAT_DIFFUSE;
         if (active)
         {
             const int2 entry = queue[qq];
             p = entry.x;
             const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
-            const V3 rayO = v3(ro.x, ro.y, ro.z), rayD = v3(rd.x, rd.y, rd.z);
-            const float lambda = ro.w;
-            const Basis lb = query_lambda(lambda, s_lam);
-            const float d65 = d65_norm(lambda, sc.d65);
+            rayO = v3(ro.x, ro.y, ro.z);
+            rayD = v3(rd.x, rd.y, rd.z);
+            lambda = ro.w;
+            lambda_pdf = rd.w;
+            lb = query_lambda(lambda, s_lam);
+            d65 = d65_norm(lambda, sc.d65);
             const uint32_t dep = ps.depths[p];
-            int depth = (int)(dep & 0xffffu);
-            int ndd = (int)(dep >> 16);
-            uint32_t fl = ps.flags[p];
-            Media media = media_default();
+            depth = (int)(dep & 0xffffu);
+            ndd = (int)(dep >> 16);
+            fl = ps.flags[p];
             if constexpr (TRACK_MEDIA)
             {
                 const float4 mv = ps.media_v[p];
@@ -782,29 +819,19 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
                 media.obj = __float_as_int(mv.w);
                 media.depth = ps.media_depth[p];
             }
-            float radiance = ps.radiance[p];
-            float mask = ps.mask[p];
-            const bool prev_did_nee = (fl & 2u) != 0u;
-            DevRand R;
+            radiance = ps.radiance[p];
+            mask = ps.mask[p];
+            prev_did_nee = (fl & 2u) != 0u;
             R.g.state = ps.rng[p];
             R.g.inc = ar_pcg_increment(ps.pixel[p]);
 
-            const float eps = intersect_eps(ndd);
-            const int slot = entry.y;
-            Hit h;
-            h.hit = false;
-            h.obj = -1;
-            h.light = -1;
-            h.dist = 0.0f;
-            h.pos = v3(0, 0, 0);
-            h.nrm = v3(0, 0, 0);
-            h.local_pos = v3(0, 0, 0);
+            eps = intersect_eps(ndd);
+            slot = entry.y;
             if (slot != -1) hit_context(sc, slot, rayO, rayD, ps.hit_t[p], &h, &ps.hit_nrm[p]);
             if (next.x >= 0) prefetch_shade_inputs(sc, ps, next);
 
             // ---- participating medium: a free flight sampled in the medium box
             // ends the segment early with probability 1 - transmittance
-            bool scatter = false;
             if ((FEAT & AR_FEAT_MEDIUM) && sc.medium.on)
             {
                 float m0, m1;
@@ -825,9 +852,6 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
             }
 
             // ---- Trace (render.cuh:109-155)
-            BsdfSample S = bsdf_sample_default();
-            Material mat;
-            mat.shading = AR_MAT_DIFFUSE;
             if (!h.hit && !scatter && media.inside)
             {
                 S.miss_thin = true;
@@ -841,7 +865,6 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
                 S.media.inside = false;
                 S.media.vertex = h.local_pos;
             }
-            int texel = -1;
             if (h.hit)
             {
                 mat = sc.materials[h.material];
@@ -898,13 +921,16 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
             }
             media = S.media;
 
-            // ---- guided mixture sampling (render.cuh:553-638)
-            const Probe* probe = nullptr;
-            V3 maskq = v3(1.0f, 1.0f, 1.0f);
-            float pgProb = 0.0f;
-            bool mlp_on = false;           // GUIDE == 2: this vertex mixes in the network's distribution
-            const uint8_t* qcells = nullptr;  // its 64 quantised cell weights (the path's inference record)
-            float q_total = 1.0f;
+        }
+        // ---- guided mixture sampling (render.cuh:553-638)
+        const Probe* probe = nullptr;
+        V3 maskq = v3(1.0f, 1.0f, 1.0f);
+        float pgProb = 0.0f;
+        bool mlp_on = false;           // GUIDE == 2: this vertex mixes in the network's distribution
+        const uint8_t* qcells = nullptr;  // its 64 quantised cell weights (the path's inference record)
+        float q_total = 1.0f;
+        if (active)
+        {
             if constexpr (GUIDE)
             {
                 const float4 mq = ps.maskq[p];
@@ -1064,7 +1090,11 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
                                  false, rayD, h.pos, h.nrm);
             }
 
-            const bool ended = (!h.hit && !S.miss_thin && !scatter) || S.terminate;
+            ended = (!h.hit && !S.miss_thin && !scatter) || S.terminate;
+        }
+        if (SYNC_NEE) __syncthreads();
+        if (active)
+        {
             if (!ended)
             {
                 // ---- NEE (render.cuh:766-827, 206-343)
@@ -1211,7 +1241,7 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
                     {
                         keep = true;
                         ps.ray_o[p] = make_float4(h.pos.x, h.pos.y, h.pos.z, lambda);
-                        ps.ray_d[p] = make_float4(S.next_dir.x, S.next_dir.y, S.next_dir.z, rd.w);
+                        ps.ray_d[p] = make_float4(S.next_dir.x, S.next_dir.y, S.next_dir.z, lambda_pdf);
                         ps.mask[p] = mask;
                         ps.depths[p] = (uint32_t)depth | ((uint32_t)ndd << 16);
                         fl = (fl & ~1u) | (media.inside ? 1u : 0u);
