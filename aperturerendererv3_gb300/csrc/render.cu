@@ -724,6 +724,542 @@ __global__ void __launch_bounds__(AR_BLOCK) k_partition(const int* __restrict__ 
 #define AR_FEAT_ALL (AR_MATS_ALL | AR_FEAT_MEDIUM | AR_FEAT_TEX)
 #define AR_FEAT_SURFACE (AR_MATS_DIFFUSE | AR_MATS_LIGHT | AR_MATS_GGX)
 
+// The shadow ray a vertex casts for its light sample, and what it adds to the
+// path's radiance either way.
+struct ShadowRay
+{
+    bool cast = false, valid = false;
+    V3 o = v3(0, 0, 0), d = v3(0, 0, 0);
+    float tmax = 0.0f, vun = 0.0f, vocc = 0.0f, sdf_eps = 0.0f;
+};
+
+// One vertex of path p: the hit (slot, -1: none) reconstructed, the BSDF sampled,
+// emission and next-event estimation, roulette, the path's state for its next
+// ray.  Returns whether the path goes on; sh is the shadow ray to test.  Every
+// thread of the block calls it (barriers inside), those without a path with
+// active = false.  next: the entry this thread shades after this one, whose
+// state is prefetched once this one's loads have arrived (path -1: none).
+// Without glass the path never enters an object: its media record stays
+// the default and is neither read nor written.  Unguided forward renders
+// read nothing of an ended path but its radiance.
+template <int GUIDE, bool ADJ, int FEAT>
+__device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState& ps, const ShadeParams& prm,
+                                             const float* s_lam, bool active, int p, int slot, int2 next, ShadowRay& sh,
+                                             float& g_med_albedo, float& g_med_emission)
+{
+    constexpr bool TRACK_MEDIA = (FEAT & AR_MATS_GLASS) != 0;
+    constexpr bool STORE_ENDED = GUIDE != 0 || ADJ;
+    constexpr bool SYNC_NEE = FEAT != AR_FEAT_SURFACE;
+    bool keep = false;
+    // state of the vertex, across the phases below
+    V3 rayO = v3(0, 0, 0), rayD = v3(0, 0, 0);
+    float lambda = 0.0f, lambda_pdf = 0.0f, d65 = 0.0f, radiance = 0.0f, mask = 0.0f, eps = 0.0f;
+    Basis lb = {{0.0f, 0.0f, 0.0f, 0.0f}};
+    int depth = 0, ndd = 0, texel = -1;
+    uint32_t fl = 0u;
+    bool prev_did_nee = false, scatter = false, ended = true;
+    Media media = media_default();
+    DevRand R;
+    R.g.state = 0u;
+    R.g.inc = 0u;
+    Hit h;
+    h.hit = false;
+    h.obj = -1;
+    h.light = -1;
+    h.dist = 0.0f;
+    h.pos = v3(0, 0, 0);
+    h.nrm = v3(0, 0, 0);
+    h.local_pos = v3(0, 0, 0);
+    BsdfSample S = bsdf_sample_default();
+    Material mat;
+    mat.shading = AR_MAT_DIFFUSE;
+    if (active)
+    {
+        const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
+        rayO = v3(ro.x, ro.y, ro.z);
+        rayD = v3(rd.x, rd.y, rd.z);
+        lambda = ro.w;
+        lambda_pdf = rd.w;
+        lb = query_lambda(lambda, s_lam);
+        d65 = d65_norm(lambda, sc.d65);
+        const uint32_t dep = ps.depths[p];
+        depth = (int)(dep & 0xffffu);
+        ndd = (int)(dep >> 16);
+        fl = ps.flags[p];
+        if constexpr (TRACK_MEDIA)
+        {
+            const float4 mv = ps.media_v[p];
+            media.inside = (fl & 1u) != 0u;
+            media.vertex = v3(mv.x, mv.y, mv.z);
+            media.obj = __float_as_int(mv.w);
+            media.depth = ps.media_depth[p];
+        }
+        radiance = ps.radiance[p];
+        mask = ps.mask[p];
+        prev_did_nee = (fl & 2u) != 0u;
+        R.g.state = ps.rng[p];
+        R.g.inc = ar_pcg_increment(ps.pixel[p]);
+
+        eps = intersect_eps(ndd);
+        if (slot != -1) hit_context(sc, slot, rayO, rayD, ps.hit_t[p], &h, &ps.hit_nrm[p]);
+        if (next.x >= 0) prefetch_shade_inputs(sc, ps, next);
+
+        // ---- participating medium: a free flight sampled in the medium box
+        // ends the segment early with probability 1 - transmittance
+        if ((FEAT & AR_FEAT_MEDIUM) && sc.medium.on)
+        {
+            float m0, m1;
+            if (medium_segment(sc.medium, rayO, rayD, 0.0f, h.hit ? h.dist : 3.0e38f, &m0, &m1))
+            {
+                const float ts = m0 - arm_logf(R()) / sc.medium.sigma_t;
+                if (ts < m1)
+                {
+                    scatter = true;
+                    h.hit = false;
+                    h.obj = -1;
+                    h.light = -1;
+                    h.dist = ts;
+                    h.pos = rayO + rayD * ts;
+                    h.nrm = v3(0.0f, 0.0f, 0.0f);
+                }
+            }
+        }
+
+        // ---- Trace (render.cuh:109-155)
+        if (!h.hit && !scatter && media.inside)
+        {
+            S.miss_thin = true;
+            S.brdf = 1.0f;
+            S.next_dir = rayD;
+            S.pdf = 1.0f;
+            h.local_pos = rayO;
+            h.obj = media.obj;
+            S.delta = true;
+            S.emissive = v3(0, 0, 0);
+            S.media.inside = false;
+            S.media.vertex = h.local_pos;
+        }
+        if (h.hit)
+        {
+            mat = sc.materials[h.material];
+            if ((FEAT & AR_FEAT_TEX) && mat.albedo_tex >= 0 && sc.tex_count > 0)
+            {
+                texel = albedo_texel(sc, mat.albedo_tex, slot, h.obj, h.pos);
+                if (texel >= 0)
+                {
+                    const float* tx = sc.texels + 3 * (size_t)texel;
+                    mat.albedo = v3(__ldg(tx), __ldg(tx + 1), __ldg(tx + 2));
+                    mat.albedo_c = prepare_color(mat.albedo, PlainFetch{sc.lut_rgb});
+                }
+            }
+            S = evaluate_material<FEAT & AR_MATS_ALL>(lambda, lb, R, mat, rayD, h, media);
+        }
+        else if (scatter)
+        {
+            // Henyey-Greenstein phase sampling; throughput x albedo
+            const float e0 = R();
+            const float e1 = R();
+            const DirSample ph = hg_sample(e0, e1, rayD, sc.medium.g);
+            S.next_dir = ph.dir;
+            S.pdf = ph.pdf;
+            S.brdf = sc.medium.albedo * ph.pdf;
+            S.delta = false;
+            S.emissive = v3(0.0f, 0.0f, 0.0f);
+            S.media = media;
+        }
+        else
+        {
+            S.brdf = 1.0f;
+            S.delta = false;
+            S.next_dir = rayD;
+            S.pdf = 1.0f;
+            S.emissive = sky_lighting(rayD);
+            S.media.inside = false;
+        }
+        // denoiser G-buffer of the camera ray's hit (RecordScreenGBuffer at
+        // depth 0, core/render/render.cuh:640-643): albedo (texel when
+        // textured), material index (-1: no surface), normal, distance
+        if constexpr (!ADJ)
+        {
+            if (prm.gbuf && depth == 0)
+            {
+                const int mid = h.hit ? h.material : -1;
+                const V3 alb = h.hit ? mat.albedo : v3(0.0f, 0.0f, 0.0f);
+                prm.gbuf[2 * (size_t)p] = make_float4(alb.x, alb.y, alb.z, __int_as_float(mid));
+                prm.gbuf[2 * (size_t)p + 1] = make_float4(h.nrm.x, h.nrm.y, h.nrm.z, h.dist);
+            }
+        }
+        {
+            const float offsetEPS = eps * fmaxf(1.0f, length(h.pos));
+            h.pos = h.pos + signf(dot(h.nrm, S.next_dir)) * h.nrm * offsetEPS * (R() + 0.5f);
+        }
+        media = S.media;
+
+    }
+    // ---- guided mixture sampling (render.cuh:553-638)
+    const Probe* probe = nullptr;
+    V3 maskq = v3(1.0f, 1.0f, 1.0f);
+    float pgProb = 0.0f;
+    bool mlp_on = false;           // GUIDE == 2: this vertex mixes in the network's distribution
+    const uint8_t* qcells = nullptr;  // its 64 quantised cell weights (the path's inference record)
+    float q_total = 1.0f;
+    if (active)
+    {
+        if constexpr (GUIDE)
+        {
+            const float4 mq = ps.maskq[p];
+            maskq = v3(mq.x, mq.y, mq.z);
+            pgProb = guide_probability((int)ps.frame[p]);  // the path's own frame (waves may hold several)
+            const bool eligible = h.hit && !S.delta && !S.pure_light && !media.inside;
+            if constexpr (GUIDE == 2)
+            {
+                if (eligible && prm.mlp_ready && ps.q_pos[p].w > 0.0f)
+                {
+                    const uint8_t* q = ps.q_dist + 64 * (size_t)p;
+                    qcells = q;
+                    q_total = mlp_total(q);
+                    mlp_on = true;
+                    const float pB = S.pdf;
+                    const float pP = mlp_hemisphere_pdf(q, 1.0f / q_total, S.next_dir, h.nrm);
+                    if (pB > 1.0e-12f && pP > 1.0e-12f)
+                    {
+                        if (R() < pgProb)
+                        {
+                            const GuideSample g = mlp_sample_hemisphere(q, q_total, R, h.nrm);
+                            if (dot(g.dir, h.nrm) > 1.0e-12f)
+                            {
+                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
+                                S.next_dir = g.dir;
+                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
+                                S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
+                            }
+                            else
+                            {
+                                mlp_on = false;
+                            }
+                        }
+                        else
+                        {
+                            S.pdf = (1.0f - pgProb) * pB + pgProb * pP;
+                        }
+                    }
+                    else
+                    {
+                        mlp_on = false;
+                    }
+                }
+            }
+            if (!mlp_on && eligible && sc.guide.probe_count > 0)
+            {
+                const VoxelKey key = voxel_key(h.pos, reflect(rayD, h.nrm), sc.guide.inv_unit);
+                const int idx = guide_lookup(sc.guide, guide_pack(key));
+                if (idx >= 0)
+                {
+                    probe = &sc.guide.probes[idx];
+                    const float pB = S.pdf;
+                    const float pP = octahedron_hemisphere_pdf(*probe, S.next_dir, h.nrm, maskq);
+                    if (pB > 1.0e-12f && pP > 1.0e-12f)
+                    {
+                        if (R() < pgProb)
+                        {
+                            const GuideSample g = sample_octahedron_hemisphere(*probe, R, h.nrm, maskq);
+                            if (dot(g.dir, h.nrm) > 1.0e-12f)
+                            {
+                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
+                                S.next_dir = g.dir;
+                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
+                                S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
+                            }
+                            else
+                            {
+                                probe = nullptr;
+                            }
+                        }
+                        else
+                        {
+                            S.pdf = (1.0f - pgProb) * pB + pgProb * pP;
+                        }
+                    }
+                    else
+                    {
+                        probe = nullptr;
+                    }
+                }
+            }
+        }
+
+        // ---- emission (render.cuh:647-723)
+        V3 endpointLe = v3(0.0f, 0.0f, 0.0f);
+        float medium_unit = 0.0f;  // emission released at this scattering point per unit emission
+        if (scatter)
+        {
+            medium_unit = mask * (1.0f - sc.medium.albedo) * d65;
+            radiance = radiance + medium_unit * sc.medium.emission;
+        }
+        else if (!h.hit)
+        {
+            if (!S.miss_thin)
+            {
+                endpointLe = S.emissive;
+                const PlainFetch f{sc.lut_rgb};
+                radiance = radiance + mask * interact_rgb(lb, S.emissive, f) * d65;
+            }
+        }
+        else if (h.light >= 0)
+        {
+            float misW = 1.0f;
+            if (prm.use_nee && depth > 0 && prev_did_nee)
+            {
+                const float4 pv = ps.prev[p];
+                const float pB = fmaxf(pv.w, 0.0f);
+                const Light L = sc.lights[h.light];
+                float pL = 0.0f;
+                const V3 lastPos = v3(pv.x, pv.y, pv.z);
+                if (L.type == AR_OBJ_CUBE) pL = box_light_pdf_omega(sc.trav.objects[L.obj], L.select_prob, lastPos, h.pos, h.nrm);
+                else if (L.type == AR_OBJ_SPHERE) pL = sphere_light_pdf_omega(sc.trav.objects[L.obj], L.select_prob, lastPos, h.pos, h.nrm);
+                if (pL >= 0.0f && pB > 0.0f) misW = power_heuristic(pB, pL);
+            }
+            endpointLe = S.emissive * misW;
+            radiance = radiance + mask * interact(mat.emissive_c, lb) * d65 * misW;
+        }
+        else if (!all_zero(S.emissive))
+        {
+            endpointLe = S.emissive;
+        }
+        if constexpr (ADJ)
+        {
+            // replay adjoint: every contribution still to come on this path
+            // (NEE here, emission and NEE further on) carries this vertex's
+            // albedo once; radiance holds the contributions that do not
+            if (scatter && prm.grad_medium)
+            {
+                // later contributions carry this albedo once; the emission here carries (1 - albedo)
+                const float dlt = ps.adj_delta[p];
+                const float a = sc.medium.albedo;
+                const float rest = ps.adj_total[p] - radiance;
+                if (a > 1.0e-8f) g_med_albedo += dlt * rest / a;
+                // d/d albedo of (1 - albedo) x emission x mask, and d/d emission
+                g_med_albedo -= dlt * mask * sc.medium.emission * d65;
+                g_med_emission += dlt * medium_unit;
+            }
+            if (prm.grad && texel >= 0 && mat.shading == AR_MAT_DIFFUSE)
+            {
+                const float rest = ps.adj_total[p] - radiance;
+                const float dlt = ps.adj_delta[p];
+                const float alb = interact(mat.albedo_c, lb);
+                if (rest != 0.0f && dlt != 0.0f && alb > 1.0e-8f)
+                {
+                    const V3 g = interact_rgb_grad(lb, mat.albedo, PlainFetch{sc.lut_rgb}) * (dlt * rest / alb);
+                    float* gp = prm.grad + 3 * (size_t)texel;
+                    if (g.x != 0.0f) atomicAdd(gp + 0, g.x);
+                    if (g.y != 0.0f) atomicAdd(gp + 1, g.y);
+                    if (g.z != 0.0f) atomicAdd(gp + 2, g.z);
+                }
+            }
+        }
+        if constexpr (GUIDE)
+        {
+            const PlainFetch f{sc.lut_rgb};
+            collect_radiance(ps, p, fl, interact_rgb(lb, endpointLe, f) * d65, S.next_dir, 0.0f, 1.0f, ndd, false,
+                             false, rayD, h.pos, h.nrm);
+        }
+
+        ended = (!h.hit && !S.miss_thin && !scatter) || S.terminate;
+    }
+    if (SYNC_NEE) __syncthreads();
+    if (active)
+    {
+        if (!ended)
+        {
+            // ---- NEE (render.cuh:766-827, 206-343)
+            if (!S.miss_thin)
+            {
+                const float useNEERate = sqrtf(saturate(mask));
+                bool neeValid = false;
+                if (prm.use_nee && ndd < AR_NEE_MAX_NON_DELTA_DEPTH && !S.delta && !media.inside && R() < useNEERate)
+                {
+                    LightSample ls;
+                    ls.valid = false;
+                    if (sc.light_count > 0)
+                    {
+                        const float r = R();
+                        int pick = sc.light_count - 1;
+                        float pickProb = 0.0f;
+                        // first light whose running CDF exceeds r (same as the sequential scan)
+                        int lo = 0, hi = sc.light_count;
+                        while (lo < hi)
+                        {
+                            const int mid = (lo + hi) >> 1;
+                            if (r < sc.lights[mid].cdf) hi = mid;
+                            else lo = mid + 1;
+                        }
+                        if (lo < sc.light_count)
+                        {
+                            pick = lo;
+                            pickProb = sc.lights[lo].select_prob;
+                        }
+                        const Light L = sc.lights[pick];
+                        if (L.type == AR_OBJ_CUBE) ls = sample_box_light(R, sc.trav.objects[L.obj], h.pos);
+                        else if (L.type == AR_OBJ_SPHERE) ls = sample_sphere_light(R, sc.trav.objects[L.obj], h.pos);
+                        if (ls.valid)
+                        {
+                            ls.obj = L.obj;
+                            ls.material = L.material;
+                            ls.p_facet = ls.p_facet * pickProb;
+                        }
+                    }
+                    const float vZero = mask * 0.0f * d65;
+                    if (!ls.valid)
+                    {
+                        radiance = radiance + vZero;
+                    }
+                    else
+                    {
+                        const float pATotal = fmaxf(1e-20f, ls.p_a * ls.p_facet);
+                        const V3 lun = ls.point - h.pos;
+                        const float dist2 = fmaxf(dot(lun, lun), (float)1.0e-12);
+                        const V3 L = lun * arm_rsqrtf(dist2);
+                        const float cosX = scatter ? 1.0f : fmaxf(0.0f, dot(h.nrm, L));
+                        const float cosY = fmaxf(0.0f, dot(ls.normal, -L));
+                        float vUn = vZero;
+                        bool validUn = false;
+                        if (!(cosX <= 0.0f || cosY <= 0.0f))
+                        {
+                            const float brdfCos =
+                                scatter ? sc.medium.albedo * hg_pdf(dot(rayD, L), sc.medium.g)
+                                        : eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, L, h, media_default());
+                            const float G = (cosY / dist2);
+                            const float le = interact(sc.materials[ls.material].emissive_c, lb);
+                            const float contribution = brdfCos * le * (G / pATotal);
+                            const float pLight = area_to_solid_angle_pdf(h.pos, ls.point, ls.normal, ls.p_facet * ls.p_a);
+                            float pBsdf = scatter ? hg_pdf(dot(rayD, L), sc.medium.g)
+                                                  : fmaxf(bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, L), 0.0f);
+                            if constexpr (GUIDE)
+                            {
+                                if (probe)
+                                    pBsdf = (1.0f - pgProb) * pBsdf +
+                                            pgProb * octahedron_hemisphere_pdf(*probe, L, h.nrm, maskq);
+                                if (mlp_on)
+                                    pBsdf = (1.0f - pgProb) * pBsdf +
+                                            pgProb * mlp_hemisphere_pdf(qcells, 1.0f / q_total, L, h.nrm);
+                            }
+                            const float misW = power_heuristic(pLight, pBsdf);
+                            vUn = mask * (contribution * misW) * d65;
+                            if ((FEAT & AR_FEAT_MEDIUM) && sc.medium.on)
+                                vUn *= medium_transmittance(sc.medium, h.pos, L, sqrtf(dist2));
+                            validUn = true;
+                        }
+                        // shadow segment (intersection.cuh:285-310)
+                        V3 dirS = ls.point - h.pos;
+                        const float distance = length(dirS);
+                        bool traced = false;
+                        if (distance > 0.0f)
+                        {
+                            dirS = dirS / distance;
+                            const float seps = intersect_eps(depth) * fmaxf(1.0f, fmaxf(length(h.pos), length(ls.point)));
+                            const float tmax = fmaxf(0.0f, distance - seps);
+                            if (tmax > 0.0f)
+                            {
+                                traced = true;
+                                sh.cast = true;
+                                sh.o = h.pos;
+                                sh.d = dirS;
+                                sh.tmax = tmax;
+                                sh.sdf_eps = 0.5f * intersect_eps(depth);  // SDF_EPS of the NEE depth
+                                sh.vun = vUn;
+                                sh.vocc = vZero;
+                                sh.valid = validUn;
+                            }
+                        }
+                        if (!traced)
+                        {
+                            radiance = radiance + vUn;
+                            neeValid = validUn;
+                        }
+                    }
+                }
+                fl = (fl & ~2u) | (neeValid ? 2u : 0u);
+                ps.prev[p] = make_float4(h.pos.x, h.pos.y, h.pos.z, S.pdf);
+            }
+            // ---- Russian roulette (render.cuh:829-859)
+            const float contrib = S.brdf / fmaxf(S.pdf, 1e-12f);
+            float pSurvive = 1.0f;
+            bool survived = true;
+            if (ndd >= AR_MIN_TRACING_DEPTH)
+            {
+                const float basic = clampf(mask * 0.5f + mask * 0.5f, 0.05f, 0.95f);
+                pSurvive = lerpf(basic, 1.0f, media.inside ? AR_DELTA_RR_TERMINATE_REDUCE : 0.0f);
+                if (R() > pSurvive) survived = false;
+            }
+            if (survived)
+            {
+                if constexpr (GUIDE)
+                {
+                    const bool allowStart = h.hit && !S.delta && !S.pure_light && !media.inside;
+                    collect_radiance(ps, p, fl, 0.0f, S.next_dir, contrib, pSurvive, ndd, allowStart, true, rayD, h.pos,
+                                     h.nrm);
+                }
+                mask = mask * contrib;
+                mask = mask / pSurvive;
+                if constexpr (GUIDE)
+                {
+                    const V3 xyz = lambda_to_xyz(lambda, sc.cie_cmf);
+                    V3 q = vmax(mask * xyz, (float)AR_PG_QUERY_EPS);
+                    const float div = (float)((double)sum3(q) + AR_PG_QUERY_EPS);
+                    q = q / div;
+                    ps.maskq[p] = make_float4(q.x, q.y, q.z, 0.0f);
+                }
+                if (!S.delta) ++ndd;
+                ++depth;
+                if (depth < prm.max_depth)
+                {
+                    keep = true;
+                    ps.ray_o[p] = make_float4(h.pos.x, h.pos.y, h.pos.z, lambda);
+                    ps.ray_d[p] = make_float4(S.next_dir.x, S.next_dir.y, S.next_dir.z, lambda_pdf);
+                    ps.mask[p] = mask;
+                    ps.depths[p] = (uint32_t)depth | ((uint32_t)ndd << 16);
+                    fl = (fl & ~1u) | (media.inside ? 1u : 0u);
+                    if constexpr (TRACK_MEDIA)
+                    {
+                        ps.media_v[p] = make_float4(media.vertex.x, media.vertex.y, media.vertex.z,
+                                                    __int_as_float(media.obj));
+                        ps.media_depth[p] = media.depth;
+                    }
+                }
+            }
+        }
+        ps.radiance[p] = radiance;
+        if (STORE_ENDED || keep)
+        {
+            ps.flags[p] = fl;
+            ps.rng[p] = R.g.state;
+        }
+    }
+    return keep;
+}
+
+// the wavelength LUT into shared memory
+__device__ __forceinline__ void stage_lambda_lut(const DevScene& sc, float* s_lam)
+{
+    for (int i = threadIdx.x; i < AR_LAMBDA_LUT_RES * 4; i += blockDim.x) s_lam[i] = sc.lut_lambda[i];
+    __syncthreads();
+}
+
+// replay adjoint: the block's sums of the medium's parameter gradients
+__device__ __forceinline__ void add_medium_gradient(double* grad_medium, float g_med_albedo, float g_med_emission)
+{
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        g_med_albedo += __shfl_xor_sync(0xffffffffu, g_med_albedo, o);
+        g_med_emission += __shfl_xor_sync(0xffffffffu, g_med_emission, o);
+    }
+    if (lane_id() == 0 && (g_med_albedo != 0.0f || g_med_emission != 0.0f))
+    {
+        atomicAdd(grad_medium, (double)g_med_albedo);
+        atomicAdd(grad_medium + 1, (double)g_med_emission);
+    }
+}
+
 // What bounds k_shade is instruction supply: one vertex runs some 2,800
 // instructions of mostly straight-line code (45 KB), the SM holds 16 warps
 // (128 registers), and when each warp is somewhere else in that code most
@@ -748,17 +1284,10 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
     // block): deep bounces often have few or no paths left
     if ((long long)blockIdx.x * blockDim.x >= n) return;
     __shared__ float s_lam[AR_LAMBDA_LUT_RES * 4];
-    for (int i = threadIdx.x; i < AR_LAMBDA_LUT_RES * 4; i += blockDim.x) s_lam[i] = sc.lut_lambda[i];
-    __syncthreads();
+    stage_lambda_lut(sc, s_lam);
     const int stride = gridDim.x * blockDim.x;
     float g_med_albedo = 0.0f, g_med_emission = 0.0f;  // replay adjoint of the medium parameters
-    // The queue comes from k_partition: {path, hit slot}, hits first.
-    // Without glass the path never enters an object: its media record stays
-    // the default and is neither read nor written.  Unguided forward renders
-    // read nothing of an ended path but its radiance.
-    constexpr bool TRACK_MEDIA = (FEAT & AR_MATS_GLASS) != 0;
-    constexpr bool STORE_ENDED = GUIDE != 0 || ADJ;
-    constexpr bool SYNC_NEE = FEAT != AR_FEAT_SURFACE;
+    // the queue comes from k_partition: {path, hit slot}, hits first
     for (int bbase = blockIdx.x * blockDim.x; bbase < n; bbase += stride)
     {
         __syncthreads();  // the block's warps start the pass together
@@ -768,527 +1297,27 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
         // prefetched once this pass's own loads have arrived
         const int qn = qq + stride;
         const int2 next = qn < n ? queue[qn] : make_int2(-1, -1);
-        bool keep = false;
-        bool shadow = false;
-        int p = 0;
-        V3 sh_o = v3(0, 0, 0), sh_d = v3(0, 0, 0);
-        float sh_tmax = 0.0f, sh_vun = 0.0f, sh_vocc = 0.0f, sh_sdf_eps = 0.0f;
-        bool sh_valid = false;
-        // state of the vertex, across the phases below
-        V3 rayO = v3(0, 0, 0), rayD = v3(0, 0, 0);
-        float lambda = 0.0f, lambda_pdf = 0.0f, d65 = 0.0f, radiance = 0.0f, mask = 0.0f, eps = 0.0f;
-        Basis lb = {{0.0f, 0.0f, 0.0f, 0.0f}};
-        int depth = 0, ndd = 0, slot = -1, texel = -1;
-        uint32_t fl = 0u;
-        bool prev_did_nee = false, scatter = false, ended = true;
-        Media media = media_default();
-        DevRand R;
-        R.g.state = 0u;
-        R.g.inc = 0u;
-        Hit h;
-        h.hit = false;
-        h.obj = -1;
-        h.light = -1;
-        h.dist = 0.0f;
-        h.pos = v3(0, 0, 0);
-        h.nrm = v3(0, 0, 0);
-        h.local_pos = v3(0, 0, 0);
-        BsdfSample S = bsdf_sample_default();
-        Material mat;
-        mat.shading = AR_MAT_DIFFUSE;
-        if (active)
-        {
-            const int2 entry = queue[qq];
-            p = entry.x;
-            const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
-            rayO = v3(ro.x, ro.y, ro.z);
-            rayD = v3(rd.x, rd.y, rd.z);
-            lambda = ro.w;
-            lambda_pdf = rd.w;
-            lb = query_lambda(lambda, s_lam);
-            d65 = d65_norm(lambda, sc.d65);
-            const uint32_t dep = ps.depths[p];
-            depth = (int)(dep & 0xffffu);
-            ndd = (int)(dep >> 16);
-            fl = ps.flags[p];
-            if constexpr (TRACK_MEDIA)
-            {
-                const float4 mv = ps.media_v[p];
-                media.inside = (fl & 1u) != 0u;
-                media.vertex = v3(mv.x, mv.y, mv.z);
-                media.obj = __float_as_int(mv.w);
-                media.depth = ps.media_depth[p];
-            }
-            radiance = ps.radiance[p];
-            mask = ps.mask[p];
-            prev_did_nee = (fl & 2u) != 0u;
-            R.g.state = ps.rng[p];
-            R.g.inc = ar_pcg_increment(ps.pixel[p]);
-
-            eps = intersect_eps(ndd);
-            slot = entry.y;
-            if (slot != -1) hit_context(sc, slot, rayO, rayD, ps.hit_t[p], &h, &ps.hit_nrm[p]);
-            if (next.x >= 0) prefetch_shade_inputs(sc, ps, next);
-
-            // ---- participating medium: a free flight sampled in the medium box
-            // ends the segment early with probability 1 - transmittance
-            if ((FEAT & AR_FEAT_MEDIUM) && sc.medium.on)
-            {
-                float m0, m1;
-                if (medium_segment(sc.medium, rayO, rayD, 0.0f, h.hit ? h.dist : 3.0e38f, &m0, &m1))
-                {
-                    const float ts = m0 - arm_logf(R()) / sc.medium.sigma_t;
-                    if (ts < m1)
-                    {
-                        scatter = true;
-                        h.hit = false;
-                        h.obj = -1;
-                        h.light = -1;
-                        h.dist = ts;
-                        h.pos = rayO + rayD * ts;
-                        h.nrm = v3(0.0f, 0.0f, 0.0f);
-                    }
-                }
-            }
-
-            // ---- Trace (render.cuh:109-155)
-            if (!h.hit && !scatter && media.inside)
-            {
-                S.miss_thin = true;
-                S.brdf = 1.0f;
-                S.next_dir = rayD;
-                S.pdf = 1.0f;
-                h.local_pos = rayO;
-                h.obj = media.obj;
-                S.delta = true;
-                S.emissive = v3(0, 0, 0);
-                S.media.inside = false;
-                S.media.vertex = h.local_pos;
-            }
-            if (h.hit)
-            {
-                mat = sc.materials[h.material];
-                if ((FEAT & AR_FEAT_TEX) && mat.albedo_tex >= 0 && sc.tex_count > 0)
-                {
-                    texel = albedo_texel(sc, mat.albedo_tex, slot, h.obj, h.pos);
-                    if (texel >= 0)
-                    {
-                        const float* tx = sc.texels + 3 * (size_t)texel;
-                        mat.albedo = v3(__ldg(tx), __ldg(tx + 1), __ldg(tx + 2));
-                        mat.albedo_c = prepare_color(mat.albedo, PlainFetch{sc.lut_rgb});
-                    }
-                }
-                S = evaluate_material<FEAT & AR_MATS_ALL>(lambda, lb, R, mat, rayD, h, media);
-            }
-            else if (scatter)
-            {
-                // Henyey-Greenstein phase sampling; throughput x albedo
-                const float e0 = R();
-                const float e1 = R();
-                const DirSample ph = hg_sample(e0, e1, rayD, sc.medium.g);
-                S.next_dir = ph.dir;
-                S.pdf = ph.pdf;
-                S.brdf = sc.medium.albedo * ph.pdf;
-                S.delta = false;
-                S.emissive = v3(0.0f, 0.0f, 0.0f);
-                S.media = media;
-            }
-            else
-            {
-                S.brdf = 1.0f;
-                S.delta = false;
-                S.next_dir = rayD;
-                S.pdf = 1.0f;
-                S.emissive = sky_lighting(rayD);
-                S.media.inside = false;
-            }
-            // denoiser G-buffer of the camera ray's hit (RecordScreenGBuffer at
-            // depth 0, core/render/render.cuh:640-643): albedo (texel when
-            // textured), material index (-1: no surface), normal, distance
-            if constexpr (!ADJ)
-            {
-                if (prm.gbuf && depth == 0)
-                {
-                    const int mid = h.hit ? h.material : -1;
-                    const V3 alb = h.hit ? mat.albedo : v3(0.0f, 0.0f, 0.0f);
-                    prm.gbuf[2 * (size_t)p] = make_float4(alb.x, alb.y, alb.z, __int_as_float(mid));
-                    prm.gbuf[2 * (size_t)p + 1] = make_float4(h.nrm.x, h.nrm.y, h.nrm.z, h.dist);
-                }
-            }
-            {
-                const float offsetEPS = eps * fmaxf(1.0f, length(h.pos));
-                h.pos = h.pos + signf(dot(h.nrm, S.next_dir)) * h.nrm * offsetEPS * (R() + 0.5f);
-            }
-            media = S.media;
-
-        }
-        // ---- guided mixture sampling (render.cuh:553-638)
-        const Probe* probe = nullptr;
-        V3 maskq = v3(1.0f, 1.0f, 1.0f);
-        float pgProb = 0.0f;
-        bool mlp_on = false;           // GUIDE == 2: this vertex mixes in the network's distribution
-        const uint8_t* qcells = nullptr;  // its 64 quantised cell weights (the path's inference record)
-        float q_total = 1.0f;
-        if (active)
-        {
-            if constexpr (GUIDE)
-            {
-                const float4 mq = ps.maskq[p];
-                maskq = v3(mq.x, mq.y, mq.z);
-                pgProb = guide_probability((int)ps.frame[p]);  // the path's own frame (waves may hold several)
-                const bool eligible = h.hit && !S.delta && !S.pure_light && !media.inside;
-                if constexpr (GUIDE == 2)
-                {
-                    if (eligible && prm.mlp_ready && ps.q_pos[p].w > 0.0f)
-                    {
-                        const uint8_t* q = ps.q_dist + 64 * (size_t)p;
-                        qcells = q;
-                        q_total = mlp_total(q);
-                        mlp_on = true;
-                        const float pB = S.pdf;
-                        const float pP = mlp_hemisphere_pdf(q, 1.0f / q_total, S.next_dir, h.nrm);
-                        if (pB > 1.0e-12f && pP > 1.0e-12f)
-                        {
-                            if (R() < pgProb)
-                            {
-                                const GuideSample g = mlp_sample_hemisphere(q, q_total, R, h.nrm);
-                                if (dot(g.dir, h.nrm) > 1.0e-12f)
-                                {
-                                    const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
-                                    S.next_dir = g.dir;
-                                    S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
-                                    S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
-                                }
-                                else
-                                {
-                                    mlp_on = false;
-                                }
-                            }
-                            else
-                            {
-                                S.pdf = (1.0f - pgProb) * pB + pgProb * pP;
-                            }
-                        }
-                        else
-                        {
-                            mlp_on = false;
-                        }
-                    }
-                }
-                if (!mlp_on && eligible && sc.guide.probe_count > 0)
-                {
-                    const VoxelKey key = voxel_key(h.pos, reflect(rayD, h.nrm), sc.guide.inv_unit);
-                    const int idx = guide_lookup(sc.guide, guide_pack(key));
-                    if (idx >= 0)
-                    {
-                        probe = &sc.guide.probes[idx];
-                        const float pB = S.pdf;
-                        const float pP = octahedron_hemisphere_pdf(*probe, S.next_dir, h.nrm, maskq);
-                        if (pB > 1.0e-12f && pP > 1.0e-12f)
-                        {
-                            if (R() < pgProb)
-                            {
-                                const GuideSample g = sample_octahedron_hemisphere(*probe, R, h.nrm, maskq);
-                                if (dot(g.dir, h.nrm) > 1.0e-12f)
-                                {
-                                    const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
-                                    S.next_dir = g.dir;
-                                    S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
-                                    S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
-                                }
-                                else
-                                {
-                                    probe = nullptr;
-                                }
-                            }
-                            else
-                            {
-                                S.pdf = (1.0f - pgProb) * pB + pgProb * pP;
-                            }
-                        }
-                        else
-                        {
-                            probe = nullptr;
-                        }
-                    }
-                }
-            }
-
-            // ---- emission (render.cuh:647-723)
-            V3 endpointLe = v3(0.0f, 0.0f, 0.0f);
-            float medium_unit = 0.0f;  // emission released at this scattering point per unit emission
-            if (scatter)
-            {
-                medium_unit = mask * (1.0f - sc.medium.albedo) * d65;
-                radiance = radiance + medium_unit * sc.medium.emission;
-            }
-            else if (!h.hit)
-            {
-                if (!S.miss_thin)
-                {
-                    endpointLe = S.emissive;
-                    const PlainFetch f{sc.lut_rgb};
-                    radiance = radiance + mask * interact_rgb(lb, S.emissive, f) * d65;
-                }
-            }
-            else if (h.light >= 0)
-            {
-                float misW = 1.0f;
-                if (prm.use_nee && depth > 0 && prev_did_nee)
-                {
-                    const float4 pv = ps.prev[p];
-                    const float pB = fmaxf(pv.w, 0.0f);
-                    const Light L = sc.lights[h.light];
-                    float pL = 0.0f;
-                    const V3 lastPos = v3(pv.x, pv.y, pv.z);
-                    if (L.type == AR_OBJ_CUBE) pL = box_light_pdf_omega(sc.trav.objects[L.obj], L.select_prob, lastPos, h.pos, h.nrm);
-                    else if (L.type == AR_OBJ_SPHERE) pL = sphere_light_pdf_omega(sc.trav.objects[L.obj], L.select_prob, lastPos, h.pos, h.nrm);
-                    if (pL >= 0.0f && pB > 0.0f) misW = power_heuristic(pB, pL);
-                }
-                endpointLe = S.emissive * misW;
-                radiance = radiance + mask * interact(mat.emissive_c, lb) * d65 * misW;
-            }
-            else if (!all_zero(S.emissive))
-            {
-                endpointLe = S.emissive;
-            }
-            if constexpr (ADJ)
-            {
-                // replay adjoint: every contribution still to come on this path
-                // (NEE here, emission and NEE further on) carries this vertex's
-                // albedo once; radiance holds the contributions that do not
-                if (scatter && prm.grad_medium)
-                {
-                    // later contributions carry this albedo once; the emission here carries (1 - albedo)
-                    const float dlt = ps.adj_delta[p];
-                    const float a = sc.medium.albedo;
-                    const float rest = ps.adj_total[p] - radiance;
-                    if (a > 1.0e-8f) g_med_albedo += dlt * rest / a;
-                    // d/d albedo of (1 - albedo) x emission x mask, and d/d emission
-                    g_med_albedo -= dlt * mask * sc.medium.emission * d65;
-                    g_med_emission += dlt * medium_unit;
-                }
-                if (prm.grad && texel >= 0 && mat.shading == AR_MAT_DIFFUSE)
-                {
-                    const float rest = ps.adj_total[p] - radiance;
-                    const float dlt = ps.adj_delta[p];
-                    const float alb = interact(mat.albedo_c, lb);
-                    if (rest != 0.0f && dlt != 0.0f && alb > 1.0e-8f)
-                    {
-                        const V3 g = interact_rgb_grad(lb, mat.albedo, PlainFetch{sc.lut_rgb}) * (dlt * rest / alb);
-                        float* gp = prm.grad + 3 * (size_t)texel;
-                        if (g.x != 0.0f) atomicAdd(gp + 0, g.x);
-                        if (g.y != 0.0f) atomicAdd(gp + 1, g.y);
-                        if (g.z != 0.0f) atomicAdd(gp + 2, g.z);
-                    }
-                }
-            }
-            if constexpr (GUIDE)
-            {
-                const PlainFetch f{sc.lut_rgb};
-                collect_radiance(ps, p, fl, interact_rgb(lb, endpointLe, f) * d65, S.next_dir, 0.0f, 1.0f, ndd, false,
-                                 false, rayD, h.pos, h.nrm);
-            }
-
-            ended = (!h.hit && !S.miss_thin && !scatter) || S.terminate;
-        }
-        if (SYNC_NEE) __syncthreads();
-        if (active)
-        {
-            if (!ended)
-            {
-                // ---- NEE (render.cuh:766-827, 206-343)
-                if (!S.miss_thin)
-                {
-                    const float useNEERate = sqrtf(saturate(mask));
-                    bool neeValid = false;
-                    if (prm.use_nee && ndd < AR_NEE_MAX_NON_DELTA_DEPTH && !S.delta && !media.inside && R() < useNEERate)
-                    {
-                        LightSample ls;
-                        ls.valid = false;
-                        if (sc.light_count > 0)
-                        {
-                            const float r = R();
-                            int pick = sc.light_count - 1;
-                            float pickProb = 0.0f;
-                            // first light whose running CDF exceeds r (same as the sequential scan)
-                            int lo = 0, hi = sc.light_count;
-                            while (lo < hi)
-                            {
-                                const int mid = (lo + hi) >> 1;
-                                if (r < sc.lights[mid].cdf) hi = mid;
-                                else lo = mid + 1;
-                            }
-                            if (lo < sc.light_count)
-                            {
-                                pick = lo;
-                                pickProb = sc.lights[lo].select_prob;
-                            }
-                            const Light L = sc.lights[pick];
-                            if (L.type == AR_OBJ_CUBE) ls = sample_box_light(R, sc.trav.objects[L.obj], h.pos);
-                            else if (L.type == AR_OBJ_SPHERE) ls = sample_sphere_light(R, sc.trav.objects[L.obj], h.pos);
-                            if (ls.valid)
-                            {
-                                ls.obj = L.obj;
-                                ls.material = L.material;
-                                ls.p_facet = ls.p_facet * pickProb;
-                            }
-                        }
-                        const float vZero = mask * 0.0f * d65;
-                        if (!ls.valid)
-                        {
-                            radiance = radiance + vZero;
-                        }
-                        else
-                        {
-                            const float pATotal = fmaxf(1e-20f, ls.p_a * ls.p_facet);
-                            const V3 lun = ls.point - h.pos;
-                            const float dist2 = fmaxf(dot(lun, lun), (float)1.0e-12);
-                            const V3 L = lun * arm_rsqrtf(dist2);
-                            const float cosX = scatter ? 1.0f : fmaxf(0.0f, dot(h.nrm, L));
-                            const float cosY = fmaxf(0.0f, dot(ls.normal, -L));
-                            float vUn = vZero;
-                            bool validUn = false;
-                            if (!(cosX <= 0.0f || cosY <= 0.0f))
-                            {
-                                const float brdfCos =
-                                    scatter ? sc.medium.albedo * hg_pdf(dot(rayD, L), sc.medium.g)
-                                            : eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, L, h, media_default());
-                                const float G = (cosY / dist2);
-                                const float le = interact(sc.materials[ls.material].emissive_c, lb);
-                                const float contribution = brdfCos * le * (G / pATotal);
-                                const float pLight = area_to_solid_angle_pdf(h.pos, ls.point, ls.normal, ls.p_facet * ls.p_a);
-                                float pBsdf = scatter ? hg_pdf(dot(rayD, L), sc.medium.g)
-                                                      : fmaxf(bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, L), 0.0f);
-                                if constexpr (GUIDE)
-                                {
-                                    if (probe)
-                                        pBsdf = (1.0f - pgProb) * pBsdf +
-                                                pgProb * octahedron_hemisphere_pdf(*probe, L, h.nrm, maskq);
-                                    if (mlp_on)
-                                        pBsdf = (1.0f - pgProb) * pBsdf +
-                                                pgProb * mlp_hemisphere_pdf(qcells, 1.0f / q_total, L, h.nrm);
-                                }
-                                const float misW = power_heuristic(pLight, pBsdf);
-                                vUn = mask * (contribution * misW) * d65;
-                                if ((FEAT & AR_FEAT_MEDIUM) && sc.medium.on)
-                                    vUn *= medium_transmittance(sc.medium, h.pos, L, sqrtf(dist2));
-                                validUn = true;
-                            }
-                            // shadow segment (intersection.cuh:285-310)
-                            V3 dirS = ls.point - h.pos;
-                            const float distance = length(dirS);
-                            bool traced = false;
-                            if (distance > 0.0f)
-                            {
-                                dirS = dirS / distance;
-                                const float seps = intersect_eps(depth) * fmaxf(1.0f, fmaxf(length(h.pos), length(ls.point)));
-                                const float tmax = fmaxf(0.0f, distance - seps);
-                                if (tmax > 0.0f)
-                                {
-                                    traced = true;
-                                    shadow = true;
-                                    sh_o = h.pos;
-                                    sh_d = dirS;
-                                    sh_tmax = tmax;
-                                    sh_sdf_eps = 0.5f * intersect_eps(depth);  // SDF_EPS of the NEE depth
-                                    sh_vun = vUn;
-                                    sh_vocc = vZero;
-                                    sh_valid = validUn;
-                                }
-                            }
-                            if (!traced)
-                            {
-                                radiance = radiance + vUn;
-                                neeValid = validUn;
-                            }
-                        }
-                    }
-                    fl = (fl & ~2u) | (neeValid ? 2u : 0u);
-                    ps.prev[p] = make_float4(h.pos.x, h.pos.y, h.pos.z, S.pdf);
-                }
-                // ---- Russian roulette (render.cuh:829-859)
-                const float contrib = S.brdf / fmaxf(S.pdf, 1e-12f);
-                float pSurvive = 1.0f;
-                bool survived = true;
-                if (ndd >= AR_MIN_TRACING_DEPTH)
-                {
-                    const float basic = clampf(mask * 0.5f + mask * 0.5f, 0.05f, 0.95f);
-                    pSurvive = lerpf(basic, 1.0f, media.inside ? AR_DELTA_RR_TERMINATE_REDUCE : 0.0f);
-                    if (R() > pSurvive) survived = false;
-                }
-                if (survived)
-                {
-                    if constexpr (GUIDE)
-                    {
-                        const bool allowStart = h.hit && !S.delta && !S.pure_light && !media.inside;
-                        collect_radiance(ps, p, fl, 0.0f, S.next_dir, contrib, pSurvive, ndd, allowStart, true, rayD, h.pos,
-                                         h.nrm);
-                    }
-                    mask = mask * contrib;
-                    mask = mask / pSurvive;
-                    if constexpr (GUIDE)
-                    {
-                        const V3 xyz = lambda_to_xyz(lambda, sc.cie_cmf);
-                        V3 q = vmax(mask * xyz, (float)AR_PG_QUERY_EPS);
-                        const float div = (float)((double)sum3(q) + AR_PG_QUERY_EPS);
-                        q = q / div;
-                        ps.maskq[p] = make_float4(q.x, q.y, q.z, 0.0f);
-                    }
-                    if (!S.delta) ++ndd;
-                    ++depth;
-                    if (depth < prm.max_depth)
-                    {
-                        keep = true;
-                        ps.ray_o[p] = make_float4(h.pos.x, h.pos.y, h.pos.z, lambda);
-                        ps.ray_d[p] = make_float4(S.next_dir.x, S.next_dir.y, S.next_dir.z, lambda_pdf);
-                        ps.mask[p] = mask;
-                        ps.depths[p] = (uint32_t)depth | ((uint32_t)ndd << 16);
-                        fl = (fl & ~1u) | (media.inside ? 1u : 0u);
-                        if constexpr (TRACK_MEDIA)
-                        {
-                            ps.media_v[p] = make_float4(media.vertex.x, media.vertex.y, media.vertex.z,
-                                                        __int_as_float(media.obj));
-                            ps.media_depth[p] = media.depth;
-                        }
-                    }
-                }
-            }
-            ps.radiance[p] = radiance;
-            if (STORE_ENDED || keep)
-            {
-                ps.flags[p] = fl;
-                ps.rng[p] = R.g.state;
-            }
-        }
+        const int2 entry = active ? queue[qq] : make_int2(0, -1);
+        const int p = entry.x;
+        ShadowRay sh;
+        const bool keep = shade_vertex<GUIDE, ADJ, FEAT>(sc, ps, prm, s_lam, active, p, entry.y, next, sh, g_med_albedo,
+                                                        g_med_emission);
         const int nq = warp_append_slot(next_counter, keep);
         if (keep) next_queue[nq] = p;
-        const int sqi = warp_append_slot(shadow_counter, shadow);
-        if (shadow)
+        const int sqi = warp_append_slot(shadow_counter, sh.cast);
+        if (sh.cast)
         {
             sq.path[sqi] = p;
-            sq.o[sqi] = make_float4(sh_o.x, sh_o.y, sh_o.z, sh_tmax);
-            sq.d[sqi] = make_float4(sh_d.x, sh_d.y, sh_d.z, sh_vun);
-            sq.v_occ[sqi] = sh_vocc;
-            sq.valid_unocc[sqi] = sh_valid ? 1 : 0;
-            sq.sdf_eps[sqi] = sh_sdf_eps;
+            sq.o[sqi] = make_float4(sh.o.x, sh.o.y, sh.o.z, sh.tmax);
+            sq.d[sqi] = make_float4(sh.d.x, sh.d.y, sh.d.z, sh.vun);
+            sq.v_occ[sqi] = sh.vocc;
+            sq.valid_unocc[sqi] = sh.valid ? 1 : 0;
+            sq.sdf_eps[sqi] = sh.sdf_eps;
         }
     }
     if constexpr (ADJ)
     {
-        if (prm.grad_medium)
-        {
-            for (int o = 16; o > 0; o >>= 1)
-            {
-                g_med_albedo += __shfl_xor_sync(0xffffffffu, g_med_albedo, o);
-                g_med_emission += __shfl_xor_sync(0xffffffffu, g_med_emission, o);
-            }
-            if (lane_id() == 0 && (g_med_albedo != 0.0f || g_med_emission != 0.0f))
-            {
-                atomicAdd(prm.grad_medium, (double)g_med_albedo);
-                atomicAdd(prm.grad_medium + 1, (double)g_med_emission);
-            }
-        }
+        if (prm.grad_medium) add_medium_gradient(prm.grad_medium, g_med_albedo, g_med_emission);
     }
 }
 
@@ -1377,6 +1406,82 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_TRAV_MIN_BLOCKS) k_shadow(DevScen
                 }
             }
         }
+    }
+}
+
+// ---------------------------------------------------------------- whole paths
+// Small waves, and the last paths of large ones, go to their end in one launch
+// (k_finish): the four launches of a depth cost 60-70 us however few paths are
+// left, most of it launch and ramp-up, while a block that keeps its paths pays
+// only for their own rays and vertices.  The block's barriers keep its warps in
+// the same phase (k_shade's comment).  The line lies at 1024 paths per SM, two
+// resident sets: the launches per depth win above it, where a warp's early-ended
+// lanes stay empty in k_finish but are refilled by the queues.  One frame of the
+// Cornell box, depth 8, launches per depth against k_finish: 256x256 632 -> 332
+// us, 320x320 697 -> 488, 400x400 739 -> 718, 512x512 884 -> 1002.  Glass at depth 1000
+// with the switch at 1024 per SM: 413x307x8 3.56 -> 1.07 ms, 256x256 1.91 -> 0.36 ms.
+// Blocks of 256 (32 / 64 / 128: 388 / 361 / 348 us for the 256x256 frame, 328 here).
+#define AR_FINISH_BLOCK 256
+#define AR_FINISH_MIN_BLOCKS 2
+#define AR_FINISH_PATHS_PER_SM 1024
+
+// the closest hit of path p's ray in the main BVH (scenes without SDF
+// geometry): the slot, -1 for none; the distance into hit_t
+__device__ __forceinline__ int trace_path(const DevScene& sc, const PathState& ps, int p, unsigned int* err)
+{
+    const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
+    const V3 o = v3(ro.x, ro.y, ro.z), d = v3(rd.x, rd.y, rd.z);
+    const float tmin = intersect_eps((int)(ps.depths[p] >> 16));
+    const int mobj = (ps.flags[p] & 1u) ? __float_as_int(ps.media_v[p].w) : -1;
+    if (mobj >= 0)
+    {
+        // inside a medium: only the enclosing object (as in k_extend)
+        const int s = sc.prim_slot[mobj];
+        int id;
+        const float th = prim_hit<false>(sc.trav, s, make_shear(d), o, d, &id, tmin);
+        ps.hit_t[p] = th >= tmin ? th : 0.0f;
+        return th >= tmin ? s : -1;
+    }
+    const TravResult r = traverse<false>(sc.trav, o, d, tmin, __int_as_float(0x7f800000), err);
+    ps.hit_t[p] = r.t;
+    return r.slot;
+}
+
+// Every queued path to its end: the arithmetic of k_extend, k_shade and k_shadow
+// per path, in the same order.
+template <bool ADJ, int FEAT>
+__global__ void __launch_bounds__(AR_FINISH_BLOCK, AR_FINISH_MIN_BLOCKS)
+    k_finish(DevScene sc, PathState ps, const int* __restrict__ queue, const int* __restrict__ counter, ShadeParams prm,
+             unsigned int* err)
+{
+    const int n = *counter;
+    if ((long long)blockIdx.x * blockDim.x >= n) return;
+    __shared__ float s_lam[AR_LAMBDA_LUT_RES * 4];
+    stage_lambda_lut(sc, s_lam);
+    float g_med_albedo = 0.0f, g_med_emission = 0.0f;
+    for (int bbase = blockIdx.x * blockDim.x; bbase < n; bbase += gridDim.x * blockDim.x)
+    {
+        const int q = bbase + (int)threadIdx.x;
+        bool active = q < n;
+        const int p = active ? queue[q] : 0;
+        while (__syncthreads_or(active))
+        {
+            const int slot = active ? trace_path(sc, ps, p, err) : -1;
+            ShadowRay sh;
+            const bool keep = shade_vertex<0, ADJ, FEAT>(sc, ps, prm, s_lam, active, p, slot, make_int2(-1, -1), sh,
+                                                         g_med_albedo, g_med_emission);
+            if (sh.cast)
+            {
+                const bool occluded = traverse<true>(sc.trav, sh.o, sh.d, 0.0f, sh.tmax, err).slot >= 0;
+                ps.radiance[p] = ps.radiance[p] + (occluded ? sh.vocc : sh.vun);
+                if (keep) ps.flags[p] = (ps.flags[p] & ~2u) | ((occluded || sh.valid) ? 2u : 0u);
+            }
+            active = keep;
+        }
+    }
+    if constexpr (ADJ)
+    {
+        if (prm.grad_medium) add_medium_gradient(prm.grad_medium, g_med_albedo, g_med_emission);
     }
 }
 
@@ -1578,6 +1683,10 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     // bound sizes the grids of the queue-sized kernels, so deep bounces with
     // few paths left (or none, at depth limits like 1000) cost launches of a
     // few blocks instead of a wave-sized grid.
+    // k_finish covers scenes without SDF passes and without a guide; profiled
+    // renders keep the stages apart
+    const bool finish_ok = !has_sdf && !rl.guide && c.profile == 0;
+    const long long finish_paths = (long long)sms * AR_FINISH_PATHS_PER_SM;
     constexpr int K = AR_BOUNCE_LOOKAHEAD;
     long long bound = n;  // upper bound of the current depth's queue length
     for (int b = 0; b < rl.max_depth; ++b)
@@ -1590,6 +1699,19 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
             const int known = c.h_bounce_cnt[slot];  // queue length of depth b - K + 1
             if (known <= 0) break;
             bound = std::min<long long>(bound, known);
+        }
+        if (finish_ok && bound <= finish_paths)
+        {
+            // few enough paths: all of them to their end in one launch
+            const int grid_f = (int)std::min<long long>((bound + AR_FINISH_BLOCK - 1) / AR_FINISH_BLOCK,
+                                                        (long long)sms * AR_FINISH_MIN_BLOCKS);
+            const int* fq = c.d_queue[b & 1];
+            const int* fn = &cnt[AR_CNT_Q0 + (b & 1)];
+            if (rl.adjoint) k_finish<true, AR_FEAT_ALL><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
+            else if (lean) k_finish<false, AR_FEAT_SURFACE><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
+            else k_finish<false, AR_FEAT_ALL><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
+            ++L;
+            break;
         }
         const int grid_s = std::max(2 * sms, (int)((bound + AR_BLOCK * AR_SHADE_PATHS_PER_THREAD - 1) /
                                                    (AR_BLOCK * AR_SHADE_PATHS_PER_THREAD)));
