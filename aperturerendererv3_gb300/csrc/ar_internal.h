@@ -242,7 +242,7 @@ struct StageEvent
 
 // Per-path state of the wavefront integrator (structure of arrays).
 // ints in a render wave's counter array (layout: AR_CNT_* in render.cu)
-#define AR_CNT_COUNT 10
+#define AR_CNT_COUNT 12
 
 struct PathState
 {
@@ -403,6 +403,7 @@ struct Ctx
     float sdf_k = 0.0f;
     int sdf_material = -1;
     float4* d_sdf = nullptr;
+    unsigned long long* d_sdf_cells = nullptr;  // the union's cell grid
     SdfUnion sdf{};
     int sdf_id = -1;                     // primitive id of the SDF object
     BoxMedium medium{};
@@ -536,6 +537,8 @@ cudaError_t launch_scale_means(double* v, long long n, double inv, cudaStream_t 
 void free_denoise(Ctx& c);
 // SDF volume cache (sdfvol.cu)
 void free_volumes(Ctx& c);
+// the smooth union's cell grid (sdfvol.cu), from c.sdf's primitives and bounds
+cudaError_t build_sdf_cells(Ctx& c);
 // GPU BVH build (bvh_gpu.cu): same format as arbvh::build_wide_bvh; "" on success
 std::string build_wide_bvh_gpu(const std::vector<arbvh::PrimInput>& prims, arbvh::WideBVH& out, cudaStream_t s);
 // refit of the main BVH after mesh vertices moved (bvh_gpu.cu)

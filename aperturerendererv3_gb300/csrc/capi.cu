@@ -143,6 +143,7 @@ void free_scene(Ctx& c)
     free_dev(c.d_tex_info);
     free_dev(c.d_prim_uv);
     free_dev(c.d_sdf);
+    free_dev(c.d_sdf_cells);
     free_dev(c.d_sdf_params);
     free_dev(c.d_sdf_nodes);
     free_dev(c.d_sdf_bvh_slots);
@@ -1220,6 +1221,7 @@ ar_status ar_scene_build(ar_ctx* ctx)
         c.sdf.lo = v3(sdf_lo[0], sdf_lo[1], sdf_lo[2]);
         c.sdf.hi = v3(sdf_hi[0], sdf_hi[1], sdf_hi[2]);
         c.sdf_id = (int)nbvh;
+        AR_CUDA(ctx, build_sdf_cells(c));
     }
     std::vector<Material> mats(c.materials);
     AR_CUDA(ctx, alloc_dev(c.d_materials, std::max<size_t>(mats.size(), 1)));

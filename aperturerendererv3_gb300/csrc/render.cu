@@ -195,6 +195,7 @@ __device__ __forceinline__ int albedo_texel(const DevScene& sc, int tex, int slo
 #define AR_CNT_FETCH 4       // k_extend, k_shadow fetch counters
 #define AR_CNT_PEND 6        // pending SDF work of k_extend, k_shadow
 #define AR_CNT_PART 8        // k_partition: hits placed from the front, misses from the back
+#define AR_CNT_SDF 10        // k_sdf_extend, k_sdf_shadow fetch counters
 
 // ---------------------------------------------------------------- raygen
 struct CamParams
@@ -338,6 +339,25 @@ __device__ __forceinline__ bool warp_refill(int* fetch, int n, bool active, bool
     return *q < n;
 }
 
+// The same for groups of G lanes that hold one ray each: every lane of a group
+// gets the group's queue index.
+template <int G>
+__device__ __forceinline__ bool group_refill(int* fetch, int n, bool active, bool* exhausted, int* q, int min_idle)
+{
+    unsigned leaders = 1u;
+    for (int k = G; k < 32; k += G) leaders |= 1u << k;
+    const unsigned idle = __ballot_sync(0xffffffffu, !active) & leaders;
+    const int need = __popc(idle);
+    if (*exhausted || need < min_idle) return false;
+    int base = 0;
+    if (lane_id() == 0) base = atomicAdd(fetch, need);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base + need >= n) *exhausted = true;
+    if (active) return false;
+    *q = base + __popc(idle & ((1u << (lane_id() & ~(G - 1))) - 1u));
+    return *q < n;
+}
+
 // Counters a kernel zeroes for later kernels of the wave (block 0, thread 0,
 // before any other work): each is one that the kernel itself does not use and
 // that no kernel still running could use, so the per-depth counter resets need
@@ -350,6 +370,8 @@ struct CounterReset
     int* d;
     int* e = nullptr;
     int* f = nullptr;
+    int* g = nullptr;
+    int* h = nullptr;
 };
 
 __device__ __forceinline__ void reset_counters(const CounterReset& r)
@@ -362,6 +384,8 @@ __device__ __forceinline__ void reset_counters(const CounterReset& r)
         if (r.d) *r.d = 0;
         if (r.e) *r.e = 0;
         if (r.f) *r.f = 0;
+        if (r.g) *r.g = 0;
+        if (r.h) *r.h = 0;
     }
 }
 
@@ -389,81 +413,287 @@ __device__ __forceinline__ void extend_finish(const DevScene& sc, const PathStat
     ps.q_slot[q] = r.slot;
 }
 
-// The SDF pass of the closest hits (scenes with SDF geometry only): the SDF
-// objects' BVH from the main BVH's hit, then the smooth union (marched up to
-// the hit so far; it has the largest primitive id, so a hit at equal t wins),
-// and the normal of an SDF hit (central differences of the field), which
-// k_shade reads from hit_nrm.  Rays inside an SDF object test only it.
-__global__ void __launch_bounds__(AR_BLOCK) k_sdf_extend(DevScene sc, PathState ps, const int* __restrict__ queue,
-                                                       const int* __restrict__ counter)
+// What bounds the smooth union's passes is the chain of field evaluations along a
+// ray: 9-12 on average, a few hundred for rays that graze the surface, each the
+// blend of four to six primitives one after the other.  So an evaluation reads
+// the few primitives its cell can need (sdf_cell_mask; 32 primitives before),
+// two lanes share a ray and its primitives, and a warp fetches new rays as soon
+// as a quarter of its lanes have none, so that grazing rays do not hold the rest.
+// Terrain with 32 primitives in a medium, 4 samples, depth 24 (all passes and
+// shading): 1280x720 61.0 -> 18.8 ms, 640x360 28.8 -> 9.4, 160x90 14.1 -> 2.9 (the
+// smaller ones with k_finish).  At 640x360 groups of 1 / 2 / 4 / 8 lanes took
+// 13.4 / 11.8 / 11.3 / 13.2 ms, at 1280x720 22.1 / 22.2 / 24.9 / 34.3; 4 blocks per
+// SM 10.9, 3 blocks 11.3.
+#define AR_SDF_GROUP 2        // lanes per ray
+#define AR_SDF_MIN_BLOCKS 4   // blocks per SM the marches are compiled for
+#define AR_SDF_IDLE 4         // idle groups that trigger a refill
+#define AR_SDF_EVALS 4        // evaluations between refill checks
+
+// sdf_fold by a group of AR_SDF_GROUP lanes with the same p and mask: each
+// lane computes one primitive's distance, every lane folds them in order.
+__device__ __forceinline__ float sdf_fold_group(const SdfUnion& s, unsigned long long mask, V3 p)
+{
+    constexpr int G = AR_SDF_GROUP;
+    const int sub = lane_id() & (G - 1), lead = lane_id() & ~(G - 1);
+    const unsigned gm = ((1u << G) - 1u) << lead;  // the group's lanes take the same branches
+    float d = 0.0f;
+    bool first = true;
+    for (int base = 0; base < 64; base += 32)
+    {
+        uint32_t m = (uint32_t)(mask >> base);
+        while (m)
+        {
+            uint32_t mine = m, rest = m;
+#pragma unroll
+            for (int j = 0; j < G; ++j)
+            {
+                if (j == sub) mine = rest;
+                rest &= rest - 1u;
+            }
+            float di = 0.0f;
+            if (mine)
+            {
+                const int i = base + __ffs((int)mine) - 1;
+                di = sdf_prim_flat(s.prims[2 * i], s.prims[2 * i + 1], p);
+            }
+#pragma unroll
+            for (int j = 0; j < G; ++j)
+            {
+                const float dj = __shfl_sync(gm, di, lead + j);
+                if (m)
+                {
+                    d = first ? dj : sdf_blend(s, d, dj);
+                    first = false;
+                }
+                m &= m - 1u;
+            }
+        }
+    }
+    return d;
+}
+
+// A ray's march through the smooth union (sdf_march, one evaluation of the
+// field per step() so that a warp's lanes can be at different points of
+// different rays): the sign at the origin, the march, and, for a surface hit
+// that is kept, the six evaluations of its normal (sdf_normal).
+struct SdfMarch
+{
+    V3 o, d;
+    float t, t1, eps;
+    int n;          // -1: at the origin; then the march's steps; then AR_SDF_STEPS + axis sample
+    bool inside;
+    V3 g;           // the normal's differences
+    int cell = -2;  // the cell whose mask this is
+    unsigned long long mask = 0ull;
+
+    // false: the ray does not reach the union before tmax
+    __device__ bool begin(const SdfUnion& s, V3 o_, V3 d_, float eps_, float tmax)
+    {
+        float t0;
+        if (s.count <= 0 || !sdf_bounds_interval(s, o_, d_, &t0, &t1) || t0 >= tmax) return false;
+        o = o_;
+        d = d_;
+        eps = eps_;
+        t1 = fminf(t1, tmax);
+        t = fmaxf(0.0f, t0);
+        n = -1;
+        return true;
+    }
+    __device__ void begin_normal()
+    {
+        o = o + d * t;
+        n = AR_SDF_STEPS;
+    }
+    __device__ V3 point() const
+    {
+        if (n < 0) return o;
+        if (n < AR_SDF_STEPS) return o + d * t;
+        const int k = n - AR_SDF_STEPS;
+        const float h = 1.0e-4f;
+        const V3 e = v3(k < 2 ? h : 0.0f, k == 2 || k == 3 ? h : 0.0f, k >= 4 ? h : 0.0f);
+        return (k & 1) ? o - e : o + e;
+    }
+    // the field there, by this lane or by the group of lanes that holds this ray
+    // (all of them call with the same state); the mask stays while the ray is in
+    // one cell
+    template <bool GROUP>
+    __device__ float field(const SdfUnion& s)
+    {
+        const V3 p = point();
+        const int c = sdf_cell(s, p);
+        if (c != cell)
+        {
+            cell = c;
+            mask = c >= 0 ? s.cells[c] : sdf_all(s);
+        }
+        return GROUP ? sdf_fold_group(s, mask, p) : sdf_fold(s, mask, p);
+    }
+    // takes the field's value at point(): 0 goes on, 1 no crossing, 2 crossing
+    // at t, 3 the normal is complete in g
+    __device__ int take(float f)
+    {
+        if (n < 0)
+        {
+            inside = f <= 0.0f;
+            n = 0;
+            return 0;
+        }
+        if (n < AR_SDF_STEPS)
+        {
+            if (inside ? (f > 0.0f && f < eps) : (f < 0.0f && -f < eps)) return 2;
+            t += fmaxf(fabsf(f), eps * 0.5f);
+            ++n;
+            return (t > t1 || n >= AR_SDF_STEPS) ? 1 : 0;
+        }
+        const int k = n - AR_SDF_STEPS;
+        if (k == 0) g.x = f;
+        else if (k == 1) g.x = g.x - f;
+        else if (k == 2) g.y = f;
+        else if (k == 3) g.y = g.y - f;
+        else if (k == 4) g.z = f;
+        else g.z = g.z - f;
+        ++n;
+        return k == 5 ? 3 : 0;
+    }
+};
+
+// The SDF objects' part of a closest hit (slot, t: the main BVH's): their own
+// BVH, or, for a ray inside one of them (AR_SLOT_SOLO), that object alone.  A hit
+// on one replaces slot and t and leaves its normal in hit_nrm.  Returns whether
+// the smooth union is still to be marched.
+__device__ __forceinline__ bool sdf_objects_hit(const DevScene& sc, const PathState& ps, int p, V3 o, V3 d, float tmin,
+                                                int& slot, float& t)
+{
+    const float seps = 0.5f * fmaxf(tmin, 1.0e-3f);
+    int obj_slot = -1;  // slot in the SDF objects' BVH
+    const bool solo = slot == AR_SLOT_SOLO;
+    if (solo)
+    {
+        const int s = sc.prim_slot[__float_as_int(ps.media_v[p].w)];
+        int id;
+        const float th = prim_hit<true>(sc.sdf_trav, s, make_shear(d), o, d, &id, tmin, seps);
+        slot = -1;
+        t = 0.0f;
+        if (th >= tmin)
+        {
+            obj_slot = s;
+            t = th;
+        }
+    }
+    else if (sc.sdf_trav.node_count > 0)
+    {
+        TravResult r;
+        r.slot = slot;
+        r.t = slot >= 0 ? t : __int_as_float(0x7f800000);
+        r.id = slot >= 0 ? (int)(__float_as_uint(sc.trav.slots[3 * (size_t)slot].w) & AR_PRIM_ID_MASK) : -1;
+        const TravResult r2 = sdf_bvh_trace<false>(sc.sdf_trav, o, d, tmin, __int_as_float(0x7f800000), seps, r);
+        if (r2.id != r.id)
+        {
+            obj_slot = r2.slot;
+            t = r2.t;
+        }
+    }
+    if (obj_slot >= 0)
+    {
+        const int id = (int)(__float_as_uint(sc.sdf_trav.slots[3 * (size_t)obj_slot].w) & AR_PRIM_ID_MASK);
+        const Object ob = sc.trav.objects[id];
+        const V3 lo = mul(ob.w2o, o - ob.center);
+        const V3 ld = normalize(mul(ob.w2o, d));
+        const V3 nn = sdf_obj_normal(sdf_obj_field(sc.trav, ob, id), ob.extent, ob.o2w, lo + ld * t, seps);
+        ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+        slot = AR_SLOT_SDFOBJ_BASE - obj_slot;
+    }
+    return !solo;
+}
+
+// whether an SDF object lies on the shadow segment
+__device__ __forceinline__ bool sdf_objects_occlude(const DevScene& sc, V3 o, V3 d, float tmax, float sdf_eps)
+{
+    if (sc.sdf_trav.node_count <= 0) return false;
+    TravResult r;
+    r.t = tmax;
+    r.slot = -1;
+    r.id = -1;
+    return sdf_bvh_trace<true>(sc.sdf_trav, o, d, 0.0f, tmax, sdf_eps, r).slot >= 0;
+}
+
+// The SDF objects' pass of the closest hits (scenes with SDF objects only).
+__global__ void __launch_bounds__(AR_BLOCK) k_sdf_objects(DevScene sc, PathState ps, const int* __restrict__ queue,
+                                                        const int* __restrict__ counter)
 {
     const int n = *counter;
     for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
     {
         const int p = queue[q];
         const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
-        const V3 o = v3(ro.x, ro.y, ro.z), d = v3(rd.x, rd.y, rd.z);
-        const float tmin = intersect_eps((int)(ps.depths[p] >> 16));
-        const float seps = 0.5f * fmaxf(tmin, 1.0e-3f);
         int slot = ps.hit_slot[p];
         float t = ps.hit_t[p];
-        int sdf_obj_slot = -1;  // slot in the SDF objects' BVH of an SDF object hit
-        if (slot == AR_SLOT_SOLO)
-        {
-            const int s = sc.prim_slot[__float_as_int(ps.media_v[p].w)];
-            int id;
-            const float th = prim_hit<true>(sc.sdf_trav, s, make_shear(d), o, d, &id, tmin, seps);
-            slot = -1;
-            t = 0.0f;
-            if (th >= tmin)
-            {
-                sdf_obj_slot = s;
-                t = th;
-            }
-        }
-        else
-        {
-            TravResult r;
-            r.slot = slot;
-            r.t = slot >= 0 ? t : __int_as_float(0x7f800000);
-            r.id = slot >= 0 ? (int)(__float_as_uint(sc.trav.slots[3 * (size_t)slot].w) & AR_PRIM_ID_MASK) : -1;
-            const TravResult r2 = sdf_bvh_trace<false>(sc.sdf_trav, o, d, tmin, __int_as_float(0x7f800000), seps, r);
-            if (r2.id != r.id)
-            {
-                sdf_obj_slot = r2.slot;
-                slot = -1;
-                t = r2.t;
-            }
-            const bool any = slot >= 0 || sdf_obj_slot >= 0;
-            if (sc.trav.sdf.count > 0)
-            {
-                const float ts = sdf_march(sc.trav.sdf, o, d, sdf_eps(tmin), any ? t : 3.0e38f);
-                if (ts >= tmin && (!any || ts < t))
-                {
-                    t = ts;
-                    slot = AR_SLOT_SDF;
-                    sdf_obj_slot = -1;
-                }
-            }
-        }
-        if (slot == AR_SLOT_SDF)
-        {
-            const V3 nn = sdf_normal(sc.trav.sdf, o + d * t, 1.0e-4f);
-            ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
-        }
-        else if (sdf_obj_slot >= 0)
-        {
-            const int id = (int)(__float_as_uint(sc.sdf_trav.slots[3 * (size_t)sdf_obj_slot].w) & AR_PRIM_ID_MASK);
-            const Object ob = sc.trav.objects[id];
-            const V3 lo = mul(ob.w2o, o - ob.center);
-            const V3 ld = normalize(mul(ob.w2o, d));
-            const V3 nn = sdf_obj_normal(sdf_obj_field(sc.trav, ob, id), ob.extent, ob.o2w, lo + ld * t, seps);
-            ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
-            slot = AR_SLOT_SDFOBJ_BASE - sdf_obj_slot;
-        }
+        sdf_objects_hit(sc, ps, p, v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z),
+                        intersect_eps((int)(ps.depths[p] >> 16)), slot, t);
         ps.hit_t[p] = t;
         ps.hit_slot[p] = slot;
         ps.q_slot[q] = slot;
+    }
+}
+
+// The smooth union's pass of the closest hits: marched up to the hit so far (it
+// has the largest primitive id, so a hit at equal t wins), and the normal of a
+// hit (central differences of the field), which k_shade reads from hit_nrm.
+// Rays inside an SDF object test only that object (objects: null without any).
+__global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
+    k_sdf_extend(SdfUnion un, const Object* __restrict__ objects, PathState ps, const int* __restrict__ queue,
+                 const int* __restrict__ counter, int* fetch)
+{
+    const int n = *counter;
+    SdfMarch m;
+    m.n = 0;
+    int p = 0, q = 0, slot = -1;
+    float t = 0.0f, tmin = 0.0f;
+    bool active = false, exhausted = false;
+    while (true)
+    {
+        if (group_refill<AR_SDF_GROUP>(fetch, n, active, &exhausted, &q, AR_SDF_IDLE))
+        {
+            p = queue[q];
+            const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
+            tmin = intersect_eps((int)(ps.depths[p] >> 16));
+            slot = ps.hit_slot[p];
+            t = ps.hit_t[p];
+            const int mobj = objects && (ps.flags[p] & 1u) ? __float_as_int(ps.media_v[p].w) : -1;
+            const bool solo = mobj >= 0 && objects[mobj].type == AR_OBJ_SDF;
+            active = !solo && m.begin(un, v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z), sdf_eps(tmin),
+                                      slot != -1 ? t : 3.0e38f);
+        }
+        if (__ballot_sync(0xffffffffu, active) == 0)
+        {
+            if (exhausted) break;
+            continue;
+        }
+        if (active)
+        {
+            for (int it = 0; it < AR_SDF_EVALS; ++it)
+            {
+                const int r = m.take(m.field<true>(un));
+                if (r == 0) continue;
+                if (r == 2 && m.t >= tmin && (slot == -1 || m.t < t))
+                {
+                    t = m.t;
+                    m.begin_normal();
+                    continue;
+                }
+                if (r == 3)
+                {
+                    // every lane of the group stores the same values
+                    const V3 nn = normalize(m.g);
+                    ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                    ps.hit_t[p] = t;
+                    ps.hit_slot[p] = AR_SLOT_SDF;
+                    ps.q_slot[q] = AR_SLOT_SDF;
+                }
+                active = false;
+                break;
+            }
+        }
     }
 }
 
@@ -742,14 +972,13 @@ struct ShadowRay
 // Without glass the path never enters an object: its media record stays
 // the default and is neither read nor written.  Unguided forward renders
 // read nothing of an ended path but its radiance.
-template <int GUIDE, bool ADJ, int FEAT>
+template <int GUIDE, bool ADJ, int FEAT, bool SYNC_NEE>
 __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState& ps, const ShadeParams& prm,
                                              const float* s_lam, bool active, int p, int slot, int2 next, ShadowRay& sh,
                                              float& g_med_albedo, float& g_med_emission)
 {
     constexpr bool TRACK_MEDIA = (FEAT & AR_MATS_GLASS) != 0;
     constexpr bool STORE_ENDED = GUIDE != 0 || ADJ;
-    constexpr bool SYNC_NEE = FEAT != AR_FEAT_SURFACE;
     bool keep = false;
     // state of the vertex, across the phases below
     V3 rayO = v3(0, 0, 0), rayD = v3(0, 0, 0);
@@ -1300,8 +1529,8 @@ __global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
         const int2 entry = active ? queue[qq] : make_int2(0, -1);
         const int p = entry.x;
         ShadowRay sh;
-        const bool keep = shade_vertex<GUIDE, ADJ, FEAT>(sc, ps, prm, s_lam, active, p, entry.y, next, sh, g_med_albedo,
-                                                        g_med_emission);
+        const bool keep = shade_vertex<GUIDE, ADJ, FEAT, FEAT != AR_FEAT_SURFACE>(sc, ps, prm, s_lam, active, p, entry.y, next, sh,
+                                                                               g_med_albedo, g_med_emission);
         const int nq = warp_append_slot(next_counter, keep);
         if (keep) next_queue[nq] = p;
         const int sqi = warp_append_slot(shadow_counter, sh.cast);
@@ -1343,28 +1572,61 @@ __device__ __forceinline__ void shadow_finish(const DevScene& sc, const PathStat
     else shadow_apply(ps, sq, i, p, occluded);
 }
 
-// the SDF pass of the shadow rays the main BVH left unoccluded
-__global__ void __launch_bounds__(AR_BLOCK) k_sdf_shadow(DevScene sc, PathState ps, ShadowQueue sq, SdfPending pend)
+// The SDF passes of the shadow rays the main BVH left unoccluded: the SDF
+// objects (rays they block leave the list as -1), then the smooth union.
+__global__ void __launch_bounds__(AR_BLOCK) k_sdf_objects_shadow(DevScene sc, PathState ps, ShadowQueue sq, SdfPending pend)
 {
     const int n = *pend.count;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
     {
         const int i = pend.list[k];
-        const int p = sq.path[i];
         const float4 o4 = sq.o[i], d4 = sq.d[i];
-        const V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
-        const float tmax = o4.w;
-        TravResult r;
-        r.t = tmax;
-        r.slot = -1;
-        r.id = -1;
-        bool occluded = sdf_bvh_trace<true>(sc.sdf_trav, o, d, 0.0f, tmax, sq.sdf_eps[i], r).slot >= 0;
-        if (!occluded && sc.trav.sdf.count > 0)
+        const bool occluded =
+            sdf_objects_occlude(sc, v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z), o4.w, sq.sdf_eps[i]);
+        if (occluded || sc.trav.sdf.count <= 0) shadow_apply(ps, sq, i, sq.path[i], occluded);
+        if (occluded) pend.list[k] = -1;
+    }
+}
+
+__global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
+    k_sdf_shadow(SdfUnion un, PathState ps, ShadowQueue sq, SdfPending pend, int* fetch)
+{
+    const int n = *pend.count;
+    const bool lead = (lane_id() & (AR_SDF_GROUP - 1)) == 0;  // the group's lane that stores
+    SdfMarch m;
+    m.n = 0;
+    int i = 0, q = 0;
+    float tmax = 0.0f;
+    bool active = false, exhausted = false;
+    while (true)
+    {
+        if (group_refill<AR_SDF_GROUP>(fetch, n, active, &exhausted, &q, AR_SDF_IDLE))
         {
-            const float ts = sdf_march(sc.trav.sdf, o, d, sdf_eps(0.0f), tmax);
-            occluded = ts >= 0.0f && ts < tmax;
+            i = pend.list[q];
+            if (i >= 0)
+            {
+                const float4 o4 = sq.o[i], d4 = sq.d[i];
+                tmax = o4.w;
+                active = m.begin(un, v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z), sdf_eps(0.0f), tmax);
+                if (!active && lead) shadow_apply(ps, sq, i, sq.path[i], false);
+            }
         }
-        shadow_apply(ps, sq, i, p, occluded);
+        if (__ballot_sync(0xffffffffu, active) == 0)
+        {
+            if (exhausted) break;
+            continue;
+        }
+        if (active)
+        {
+            for (int it = 0; it < AR_SDF_EVALS; ++it)
+            {
+                const int r = m.take(m.field<true>(un));
+                if (r == 0) continue;
+                if (lead) shadow_apply(ps, sq, i, sq.path[i], r == 2 && m.t >= 0.0f && m.t < tmax);
+                active = false;
+                break;
+            }
+        }
     }
 }
 
@@ -1424,32 +1686,88 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_TRAV_MIN_BLOCKS) k_shadow(DevScen
 #define AR_FINISH_BLOCK 256
 #define AR_FINISH_MIN_BLOCKS 2
 #define AR_FINISH_PATHS_PER_SM 1024
+// With SDF geometry every depth waits for its longest marches, twice, so the line
+// lies higher: 640x360x4 (terrain, SDF, medium) 10.1 / 10.0 / 9.4 ms with the switch
+// at 1024 / 2048 / 4096 paths per SM (all of it in k_finish: 21.9), 160x90x4 8.3 ms
+// by depth and 2.9 in k_finish.  There the warps run apart: a barrier would make
+// each block wait for its longest march.
+#define AR_FINISH_SDF_PATHS_PER_SM 4096
 
-// the closest hit of path p's ray in the main BVH (scenes without SDF
-// geometry): the slot, -1 for none; the distance into hit_t
+// The closest hit of path p's ray: the slot, -1 for none; the distance into
+// hit_t, an SDF hit's normal into hit_nrm.
+template <bool SDF>
 __device__ __forceinline__ int trace_path(const DevScene& sc, const PathState& ps, int p, unsigned int* err)
 {
     const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
     const V3 o = v3(ro.x, ro.y, ro.z), d = v3(rd.x, rd.y, rd.z);
     const float tmin = intersect_eps((int)(ps.depths[p] >> 16));
     const int mobj = (ps.flags[p] & 1u) ? __float_as_int(ps.media_v[p].w) : -1;
+    int slot;
+    float t;
     if (mobj >= 0)
     {
         // inside a medium: only the enclosing object (as in k_extend)
-        const int s = sc.prim_slot[mobj];
-        int id;
-        const float th = prim_hit<false>(sc.trav, s, make_shear(d), o, d, &id, tmin);
-        ps.hit_t[p] = th >= tmin ? th : 0.0f;
-        return th >= tmin ? s : -1;
+        if (SDF && sc.trav.objects[mobj].type == AR_OBJ_SDF)
+        {
+            slot = AR_SLOT_SOLO;
+            t = 0.0f;
+        }
+        else
+        {
+            const int s = sc.prim_slot[mobj];
+            int id;
+            const float th = prim_hit<false>(sc.trav, s, make_shear(d), o, d, &id, tmin);
+            t = th >= tmin ? th : 0.0f;
+            slot = th >= tmin ? s : -1;
+        }
     }
-    const TravResult r = traverse<false>(sc.trav, o, d, tmin, __int_as_float(0x7f800000), err);
-    ps.hit_t[p] = r.t;
-    return r.slot;
+    else
+    {
+        const TravResult r = traverse<false>(sc.trav, o, d, tmin, __int_as_float(0x7f800000), err);
+        t = r.t;
+        slot = r.slot;
+    }
+    if (SDF && sdf_objects_hit(sc, ps, p, o, d, tmin, slot, t))
+    {
+        SdfMarch m;
+        if (m.begin(sc.trav.sdf, o, d, sdf_eps(tmin), slot != -1 ? t : 3.0e38f))
+        {
+            int r;
+            while ((r = m.take(m.field<false>(sc.trav.sdf))) == 0 || (r == 2 && m.t >= tmin && (slot == -1 || m.t < t)))
+                if (r == 2)
+                {
+                    t = m.t;
+                    m.begin_normal();
+                }
+            if (r == 3)
+            {
+                const V3 nn = normalize(m.g);
+                ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                slot = AR_SLOT_SDF;
+            }
+        }
+    }
+    ps.hit_t[p] = t;
+    return slot;
+}
+
+// whether a vertex's shadow ray is blocked
+template <bool SDF>
+__device__ __forceinline__ bool shadow_path(const DevScene& sc, const ShadowRay& sh, unsigned int* err)
+{
+    if (traverse<true>(sc.trav, sh.o, sh.d, 0.0f, sh.tmax, err).slot >= 0) return true;
+    if (!SDF) return false;
+    if (sdf_objects_occlude(sc, sh.o, sh.d, sh.tmax, sh.sdf_eps)) return true;
+    SdfMarch m;
+    if (!m.begin(sc.trav.sdf, sh.o, sh.d, sdf_eps(0.0f), sh.tmax)) return false;
+    int r;
+    while ((r = m.take(m.field<false>(sc.trav.sdf))) == 0) {}
+    return r == 2 && m.t >= 0.0f && m.t < sh.tmax;
 }
 
 // Every queued path to its end: the arithmetic of k_extend, k_shade and k_shadow
 // per path, in the same order.
-template <bool ADJ, int FEAT>
+template <bool ADJ, int FEAT, bool SDF>
 __global__ void __launch_bounds__(AR_FINISH_BLOCK, AR_FINISH_MIN_BLOCKS)
     k_finish(DevScene sc, PathState ps, const int* __restrict__ queue, const int* __restrict__ counter, ShadeParams prm,
              unsigned int* err)
@@ -1464,15 +1782,15 @@ __global__ void __launch_bounds__(AR_FINISH_BLOCK, AR_FINISH_MIN_BLOCKS)
         const int q = bbase + (int)threadIdx.x;
         bool active = q < n;
         const int p = active ? queue[q] : 0;
-        while (__syncthreads_or(active))
+        while (SDF ? __any_sync(0xffffffffu, active) : __syncthreads_or(active))
         {
-            const int slot = active ? trace_path(sc, ps, p, err) : -1;
+            const int slot = active ? trace_path<SDF>(sc, ps, p, err) : -1;
             ShadowRay sh;
-            const bool keep = shade_vertex<0, ADJ, FEAT>(sc, ps, prm, s_lam, active, p, slot, make_int2(-1, -1), sh,
-                                                         g_med_albedo, g_med_emission);
+            const bool keep = shade_vertex<0, ADJ, FEAT, !SDF && FEAT != AR_FEAT_SURFACE>(
+                sc, ps, prm, s_lam, active, p, slot, make_int2(-1, -1), sh, g_med_albedo, g_med_emission);
             if (sh.cast)
             {
-                const bool occluded = traverse<true>(sc.trav, sh.o, sh.d, 0.0f, sh.tmax, err).slot >= 0;
+                const bool occluded = shadow_path<SDF>(sc, sh, err);
                 ps.radiance[p] = ps.radiance[p] + (occluded ? sh.vocc : sh.vun);
                 if (keep) ps.flags[p] = (ps.flags[p] & ~2u) | ((occluded || sh.valid) ? 2u : 0u);
             }
@@ -1609,6 +1927,23 @@ static CamParams make_camera(const RenderLaunch& rl)
     return c;
 }
 
+// the SDF passes after k_extend and after k_shadow: objects, then the union
+static void launch_sdf_extend(const DevScene& sc, const PathState& ps, const int* queue, const int* qn, int* cnt,
+                              int grid_s, int grid_m, cudaStream_t s)
+{
+    if (sc.sdf_trav.node_count > 0) k_sdf_objects<<<grid_s, AR_BLOCK, 0, s>>>(sc, ps, queue, qn);
+    if (sc.trav.sdf.count > 0)
+        k_sdf_extend<<<grid_m, AR_BLOCK, 0, s>>>(sc.trav.sdf, sc.sdf_trav.node_count > 0 ? sc.trav.objects : nullptr, ps,
+                                                 queue, qn, &cnt[AR_CNT_SDF]);
+}
+
+static void launch_sdf_shadow(const DevScene& sc, const PathState& ps, const ShadowQueue& sq, const SdfPending& pend,
+                              int* cnt, int grid_s, int grid_m, cudaStream_t s)
+{
+    if (sc.sdf_trav.node_count > 0) k_sdf_objects_shadow<<<grid_s, AR_BLOCK, 0, s>>>(sc, ps, sq, pend);
+    if (sc.trav.sdf.count > 0) k_sdf_shadow<<<grid_m, AR_BLOCK, 0, s>>>(sc.trav.sdf, ps, sq, pend, &cnt[AR_CNT_SDF + 1]);
+}
+
 // records a stage interval when profiling
 struct StageScope
 {
@@ -1647,7 +1982,7 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     // the persistent traversal kernels launch as many blocks as stay
     // resident: they fetch rays from a counter, so extra blocks would only add
     // launch cost (most deep bounces have few or no paths left)
-    const int grid_t = sms * AR_TRAV_MIN_BLOCKS;
+    const int grid_t = sms * AR_TRAV_MIN_BLOCKS, grid_m = sms * AR_SDF_MIN_BLOCKS;
     int* cnt = c.d_counters;  // AR_CNT_* layout
     const CamParams cam = make_camera(rl);
     // opaque surfaces only: the shading instantiation without glass, medium and texture code
@@ -1674,6 +2009,7 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     net.box = c.mlp_box;
     // SDF geometry: its work leaves the traversal kernels for k_sdf_extend / k_sdf_shadow
     const bool has_sdf = c.sdf_object_count > 0 || c.sdf.count > 0;
+    const int n_sdf = (sc.sdf_trav.node_count > 0 ? 1 : 0) + (sc.trav.sdf.count > 0 ? 1 : 0);  // launches of each pass
     const SdfPending pend_shd{has_sdf ? c.d_pend_list : nullptr, &cnt[AR_CNT_PEND]};
     // Each depth's next-queue length is copied to pinned host memory behind
     // the depth's launches.  The host stays AR_BOUNCE_LOOKAHEAD depths ahead of
@@ -1685,8 +2021,8 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     // few blocks instead of a wave-sized grid.
     // k_finish covers scenes without SDF passes and without a guide; profiled
     // renders keep the stages apart
-    const bool finish_ok = !has_sdf && !rl.guide && c.profile == 0;
-    const long long finish_paths = (long long)sms * AR_FINISH_PATHS_PER_SM;
+    const bool finish_ok = !rl.guide && c.profile == 0;
+    const long long finish_paths = (long long)sms * (has_sdf ? AR_FINISH_SDF_PATHS_PER_SM : AR_FINISH_PATHS_PER_SM);
     constexpr int K = AR_BOUNCE_LOOKAHEAD;
     long long bound = n;  // upper bound of the current depth's queue length
     for (int b = 0; b < rl.max_depth; ++b)
@@ -1707,9 +2043,11 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
                                                         (long long)sms * AR_FINISH_MIN_BLOCKS);
             const int* fq = c.d_queue[b & 1];
             const int* fn = &cnt[AR_CNT_Q0 + (b & 1)];
-            if (rl.adjoint) k_finish<true, AR_FEAT_ALL><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
-            else if (lean) k_finish<false, AR_FEAT_SURFACE><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
-            else k_finish<false, AR_FEAT_ALL><<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
+            const auto finish = has_sdf ? (rl.adjoint ? k_finish<true, AR_FEAT_ALL, true> : k_finish<false, AR_FEAT_ALL, true>)
+                                : rl.adjoint ? k_finish<true, AR_FEAT_ALL, false>
+                                : lean       ? k_finish<false, AR_FEAT_SURFACE, false>
+                                             : k_finish<false, AR_FEAT_ALL, false>;
+            finish<<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
             ++L;
             break;
         }
@@ -1720,7 +2058,8 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
         // k_extend zeroes the next queue, shadow queue, shadow fetch and pending
         // counters; k_shadow zeroes the next k_extend's fetch counter
         const CounterReset ext_rs{&cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], &cnt[AR_CNT_FETCH + 1],
-                                  &cnt[AR_CNT_PEND], &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1]};
+                                  &cnt[AR_CNT_PEND], &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1],
+                                  &cnt[AR_CNT_SDF], &cnt[AR_CNT_SDF + 1]};
         const CounterReset shd_rs{&cnt[AR_CNT_FETCH], nullptr, nullptr, nullptr};
         {
             StageScope st(c, ST_EXTEND);
@@ -1728,8 +2067,8 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
                                                  b == 0 ? AR_EXT_REFILL_MIN0 : AR_EXT_REFILL_MIN, ext_rs);
             if (has_sdf)
             {
-                k_sdf_extend<<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.d_queue[cur], qn);
-                ++L;
+                launch_sdf_extend(sc, c.ps, c.d_queue[cur], qn, cnt, grid_s, grid_m, s);
+                L += n_sdf;
             }
         }
         {
@@ -1767,8 +2106,8 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
                                                  c.d_err, b == 0 ? AR_SHD_REFILL_MIN0 : AR_SHD_REFILL_MIN, shd_rs);
             if (has_sdf)
             {
-                k_sdf_shadow<<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pend_shd);
-                ++L;
+                launch_sdf_shadow(sc, c.ps, c.sq, pend_shd, cnt, grid_s, grid_m, s);
+                L += n_sdf;
             }
         }
         L += 3;
@@ -1806,7 +2145,7 @@ cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int grid_n = (n + AR_BLOCK - 1) / AR_BLOCK;
-    const int grid_t = sms * AR_TRAV_MIN_BLOCKS;
+    const int grid_t = sms * AR_TRAV_MIN_BLOCKS, grid_m = sms * AR_SDF_MIN_BLOCKS;
     const int grid_s = std::max(2 * sms, (n + AR_BLOCK * AR_SHADE_PATHS_PER_THREAD - 1) / (AR_BLOCK * AR_SHADE_PATHS_PER_THREAD));
     int* cnt = wb.counters;  // AR_CNT_* layout
     const CamParams cam = make_camera(rl);
@@ -1826,18 +2165,20 @@ cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb
     {
         const int cur = b & 1, nxt = cur ^ 1;
         const CounterReset ext_rs{&cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], &cnt[AR_CNT_FETCH + 1],
-                                  &cnt[AR_CNT_PEND], &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1]};
+                                  &cnt[AR_CNT_PEND], &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1],
+                                  &cnt[AR_CNT_SDF], &cnt[AR_CNT_SDF + 1]};
         const CounterReset shd_rs{&cnt[AR_CNT_FETCH], nullptr, nullptr, nullptr};
         k_extend<<<grid_t, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.queue[cur], &cnt[AR_CNT_Q0 + cur], &cnt[AR_CNT_FETCH], err,
                                              b == 0 ? AR_EXT_REFILL_MIN0 : AR_EXT_REFILL_MIN, ext_rs);
-        if (has_sdf) k_sdf_extend<<<grid_s, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.queue[cur], &cnt[AR_CNT_Q0 + cur]);
+        if (has_sdf)
+            launch_sdf_extend(sc, wb.ps, wb.queue[cur], &cnt[AR_CNT_Q0 + cur], cnt, grid_s, grid_m, s);
         k_partition<<<grid_s, AR_BLOCK, 0, s>>>(wb.queue[cur], wb.ps.q_slot, &cnt[AR_CNT_Q0 + cur], wb.pq,
                                                 &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1]);
         k_shade<0, false><<<grid_s, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, wb.pq, &cnt[AR_CNT_Q0 + cur],
                                                    wb.queue[nxt], &cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], prm);
         k_shadow<<<grid_t, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, &cnt[AR_CNT_SHADOW], &cnt[AR_CNT_FETCH + 1], pend_shd, err,
                                              b == 0 ? AR_SHD_REFILL_MIN0 : AR_SHD_REFILL_MIN, shd_rs);
-        if (has_sdf) k_sdf_shadow<<<grid_s, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, pend_shd);
+        if (has_sdf) launch_sdf_shadow(sc, wb.ps, wb.sq, pend_shd, cnt, grid_s, grid_m, s);
     }
     k_finalize<<<grid_n, AR_BLOCK, 0, s>>>(sc, wb.ps, n, nullptr);
     const long long npix = (long long)rl.width * rl.height;

@@ -14,6 +14,48 @@
 
 namespace ar
 {
+// The smooth union's cells, one thread each: cubes of 1/96 of the union's longest
+// side (at most 7 MB).  The finer the cells, the fewer primitives each one lists
+// (near the surface of 32 blobs 8.0 / 6.1 / 5.2 at 32 / 64 / 128 cells); on the
+// 640x360x4 terrain with SDF and medium 14.6 / 13.2 / 12.1 ms at 32 / 64 / 96 cells,
+// 128 within 2 % of 96.
+#define AR_SDF_CELLS 96
+__global__ void k_sdf_cells(SdfUnion s, V3 cell, unsigned long long* __restrict__ out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int x = i % s.res[0], y = (i / s.res[0]) % s.res[1], z = i / (s.res[0] * s.res[1]);
+    const V3 c = s.lo + v3(((float)x + 0.5f) * cell.x, ((float)y + 0.5f) * cell.y, ((float)z + 0.5f) * cell.z);
+    // half the diagonal, and a little for points that round into the next cell
+    out[i] = sdf_cell_mask(s, c, 0.5f * length(cell) * 1.001f);
+}
+
+cudaError_t build_sdf_cells(Ctx& c)
+{
+    SdfUnion& s = c.sdf;
+    s.rk = sdf_reciprocal_k(s.k);
+    const V3 ext = s.hi - s.lo;
+    const float edge = max3(ext) / (float)AR_SDF_CELLS;
+    const float e[3] = {ext.x, ext.y, ext.z};
+    float cell[3];
+    for (int k = 0; k < 3; ++k)
+    {
+        if (!(edge > 0.0f && edge < 1.0e30f)) return cudaSuccess;  // no grid: the full fold everywhere
+        s.res[k] = std::min(AR_SDF_CELLS, std::max(1, (int)std::ceil(e[k] / edge)));
+        cell[k] = e[k] / (float)s.res[k];
+    }
+    const int n = s.res[0] * s.res[1] * s.res[2];
+    cudaError_t err = cudaMalloc((void**)&c.d_sdf_cells, (size_t)n * sizeof(unsigned long long));
+    if (err != cudaSuccess) return err;
+    k_sdf_cells<<<(n + 127) / 128, 128, 0, c.stream>>>(s, v3(cell[0], cell[1], cell[2]), c.d_sdf_cells, n);
+    err = cudaGetLastError();
+    if (err != cudaSuccess) return err;
+    s.inv_cell = v3(1.0f / cell[0], 1.0f / cell[1], 1.0f / cell[2]);
+    s.cells = c.d_sdf_cells;
+    return cudaSuccess;
+}
+
+
 __global__ void k_fill_sdf_volume(float* __restrict__ out, int fn, float4 prm, int dx, int dy, int dz)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
