@@ -18,12 +18,13 @@
 #include <cstdint>
 #include <cuda_fp16.h>
 
+#include "ar_denoise_test.h"
 #include "ar_vec.h"
 
 #define AR_DN_RADIUS 7                   // Bilateral16x16<7> (core/scene.cu:341)
 #define AR_DN_MODELS 5                   // diffuse, light, glass, GGX, no hit (EShadingModel::MAT_MAX)
 #define AR_DN_NO_HIT 4
-#define AR_DN_TQ_SIZE 1024               // T_QUANTILE_LUT_SIZE (core/denoise/t_quantile.cuh:6)
+#define AR_DN_TQ_SIZE ar::kDnQuantiles
 
 namespace ar
 {
@@ -173,33 +174,22 @@ __device__ __forceinline__ DnKey dn_make_key(const DnGBuf& g, const DnStat& s, V
     const double num = (double)s.num;
     const uint32_t nm1 = s.num - 1u;
     const double invNumMinus1 = 1.0 / (double)(nm1 > 1u ? nm1 : 1u);
-    const uint32_t wm1 = s.num - 1u;
-    const float wden = (float)(wm1 > 1u ? wm1 : 1u);
+    const float wden = (float)(nm1 > 1u ? nm1 : 1u);
+    const float fnum = (float)s.num;
     for (int c = 0; c < 3; ++c)
     {
         const double m2 = (double)s.m2n[c] * num;
         const float var = (float)(m2 * invNumMinus1);
-        k.vth[c] = (float)((double)var / num);
+        const float up = var / fnum;
+        // (float)((double)var / num) is var / num rounded once: both are floats while
+        // num < 2^24, and a quotient of floats rounded to double and then to
+        // float rounds as if once (53 >= 2 * 24 + 2) unless it is subnormal.  The
+        // double division would cost more than all the rest of the key.
+        k.vth[c] = (s.num < (1u << 24) && (up > 0x1p-120f || up == 0.0f)) ? up : (float)((double)var / num);
         k.theta[c] = s.mean[c] + s.m3n[c] / 6.0f / var;
-        const float up = var / (float)s.num;
         k.up[c] = up;
         k.lo[c] = up * up / wden;
     }
     return k;
-}
-
-// LookupTQuantile005 (core/denoise/t_quantile.cuh:17-26); the float -> int
-// conversion saturates and maps NaN to 0, as the GPU's conversion does.
-__device__ __forceinline__ float dn_t_quantile(const float* tq, float nu)
-{
-    const float f = floorf(nu);
-    int i;
-    if (f != f) i = 0;
-    else if (f >= 2147483648.0f) i = 2147483647;
-    else if (f <= -2147483648.0f) i = (-2147483647 - 1);
-    else i = (int)f;
-    uint32_t idx = (i <= 0) ? 0u : (uint32_t)(i - 1);
-    if (idx > AR_DN_TQ_SIZE - 1) idx = AR_DN_TQ_SIZE - 1;
-    return tq[idx];
 }
 } // namespace ar
