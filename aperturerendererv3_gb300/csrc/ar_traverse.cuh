@@ -169,6 +169,9 @@ AR_HD bool packet_child_meets(const uint4& w0, const uint4& w1, const uint4& w2,
 #define AR_DEVERR_STACK 1u
 #define AR_DEVERR_QUEUE 2u
 
+// the slab test's margin per quantisation step (TravState::step)
+#define AR_SLAB_A (0x1p-8f + 0x1p-10f)
+
 // Reciprocal of a direction component for the slab test: a zero component takes
 // 2^96, so that 32768 times a node's 2^e / d stays finite (up to e = 15) and an
 // axis-parallel ray still tells the slabs it lies in from those beside it.
@@ -226,6 +229,15 @@ AR_HD float min3f(float a, float b, float c)
 #else
     return fminf(fminf(a, b), c);
 #endif
+}
+
+// bits of slots s to bits s ^ oct, in each byte
+AR_HD uint32_t octant_order(uint32_t m, uint32_t oct)
+{
+    if (oct & 1u) m = ((m & 0x5555u) << 1) | ((m >> 1) & 0x5555u);
+    if (oct & 2u) m = ((m & 0x3333u) << 2) | ((m >> 2) & 0x3333u);
+    if (oct & 4u) m = ((m & 0x0f0fu) << 4) | ((m >> 4) & 0x0f0fu);
+    return m;
 }
 
 // Traversal of one ray as a resumable state: init() sets it up, each step()
@@ -332,10 +344,9 @@ struct TravState
             // (octant bit clear): no min / max pairs.
             const float ax = sx * inv.x, ay = sy * inv.y, az = sz * inv.z;
             const float bx = (px - o.x) * inv.x, by = (py - o.y) * inv.y, bz = (pz - o.z) * inv.z;
-            constexpr float kA = 0x1p-8f + 0x1p-10f;
-            const float ex = fmaf(fabsf(ax), kA, fabsf(bx) * 0x1p-21f);
-            const float ey = fmaf(fabsf(ay), kA, fabsf(by) * 0x1p-21f);
-            const float ez = fmaf(fabsf(az), kA, fabsf(bz) * 0x1p-21f);
+            const float ex = fmaf(fabsf(ax), AR_SLAB_A, fabsf(bx) * 0x1p-21f);
+            const float ey = fmaf(fabsf(ay), AR_SLAB_A, fabsf(by) * 0x1p-21f);
+            const float ez = fmaf(fabsf(az), AR_SLAB_A, fabsf(bz) * 0x1p-21f);
             const float cx = fmaf(-32768.0f, ax, bx), cy = fmaf(-32768.0f, ay, by), cz = fmaf(-32768.0f, az, bz);
             const bool fx = oct & 1u, fy = oct & 2u, fz = oct & 4u;
             const uint32_t nx0 = fx ? w3.z : w2.x, nx1 = fx ? w3.w : w2.y, fx0 = fx ? w2.x : w3.z, fx1 = fx ? w2.y : w3.w;
@@ -361,10 +372,7 @@ struct TravState
                     hit |= 2u << s;
             }
             // internal children low, leaves high, then both in the ray's octant order: slot s -> s ^ oct
-            uint32_t both = (hit & imask) | ((hit & ~imask) << 8);
-            if (fx) both = ((both & 0x5555u) << 1) | ((both >> 1) & 0x5555u);
-            if (fy) both = ((both & 0x3333u) << 2) | ((both >> 2) & 0x3333u);
-            if (fz) both = ((both & 0x0f0fu) << 4) | ((both >> 4) & 0x0f0fu);
+            const uint32_t both = octant_order((hit & imask) | ((hit & ~imask) << 8), oct);
             uint32_t hit_int = both & 0xffu, hit_leaf = both >> 8;
             while (hit_leaf)
             {
