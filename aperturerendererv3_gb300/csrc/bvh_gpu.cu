@@ -316,184 +316,230 @@ struct CollapseArgs
     int node_cap;
 };
 
-// one wide node per queue entry (wide index, binary index); internal children
-// are appended to the next level's queue
-__global__ void k_collapse(CollapseArgs a, const int2* __restrict__ queue, int nq, int2* next, int* next_count,
-                           unsigned int* err)
+// Exponent e (biased by 127 in a node) of the smallest power of two with
+// 255 2^e >= hi - lo, at least 2^-126: the difference rounded up is m 2^k with m in
+// [1, 2), and 255 is 1.9921875 2^7.
+__device__ __forceinline__ int quant_exponent(float lo, float hi)
 {
-    const int qi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (qi >= nq) return;
+    const float ext = __fsub_ru(hi, lo);
+    if (!(ext > 0.0f)) return -126;
+    const uint32_t u = __float_as_uint(ext);
+    const int k = (int)(u >> 23) - 127;
+    const int e = k - 7 + ((u & 0x7fffffu) > 0x7f0000u || k == 128 ? 1 : 0);
+    return e < -126 ? -126 : e;
+}
+
+// A child plane in steps of 2^e above the node's low plane, moved outwards: the
+// difference is rounded away from the box, the scaling is exact.
+__device__ __forceinline__ uint8_t quant_low(float lo, float node_lo, float inv_step)
+{
+    return (uint8_t)fminf(fmaxf(floorf(__fsub_rd(lo, node_lo) * inv_step), 0.0f), 255.0f);
+}
+__device__ __forceinline__ uint8_t quant_high(float hi, float node_lo, float inv_step)
+{
+    return (uint8_t)fminf(fmaxf(ceilf(__fsub_ru(hi, node_lo) * inv_step), 0.0f), 255.0f);
+}
+
+// One wide node per 8 lanes, one lane per child (lane k of a group: child k, then
+// slot k).  A node by a single thread is a serial chain of some 1,500 double
+// precision operations and its local arrays; by a group it is a few rounds of
+// shuffles (200,000 triangles, 7 levels: 1068 -> 256 us).  queue: (wide index,
+// binary index); internal children are appended to the next level's queue.
+__global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __restrict__ queue, int nq, int2* next,
+                                                int* next_count, unsigned int* err)
+{
+    const int lane = threadIdx.x & 31, sub = lane & 7, lead = lane & 24;
+    const unsigned gm = 0xffu << lead;
+    const int qi = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    if (qi >= nq) return;  // whole groups
     const int wi = queue[qi].x, b = queue[qi].y;
     const int n = a.n;
-    int ch[8];
-    int nch = 0;
-    if (node_count(b, n, a.range) <= kMaxLeaf) ch[nch++] = b;
+    // children: the largest-area one that is no leaf is opened until there are 8
+    int ch = -1, nch;
+    if (node_count(b, n, a.range) <= kMaxLeaf)
+    {
+        if (sub == 0) ch = b;
+        nch = 1;
+    }
     else
     {
-        ch[nch++] = a.child[b].x;
-        ch[nch++] = a.child[b].y;
+        const int2 c = a.child[b];
+        if (sub < 2) ch = sub == 0 ? c.x : c.y;
+        nch = 2;
+    }
+    int cnt = ch >= 0 ? node_count(ch, n, a.range) : 0;
+    Box6 cb{};
+    double area = -1.0;
+    if (ch >= 0)
+    {
+        cb = a.box[ch];
+        if (cnt > kMaxLeaf) area = box_area(cb);
     }
     while (nch < 8)
     {
-        int pick = -1;
-        double best = -1.0;
-        for (int i = 0; i < nch; ++i)
+        double best = area;
+        int pick = sub;
+        for (int k = 4; k > 0; k >>= 1)
         {
-            if (node_count(ch[i], n, a.range) <= kMaxLeaf) continue;
-            const double ar = box_area(a.box[ch[i]]);
-            if (ar > best)
+            const double o = __shfl_xor_sync(gm, best, k);
+            const int p = __shfl_xor_sync(gm, pick, k);
+            if (o > best || (o == best && p < pick))
             {
-                best = ar;
-                pick = i;
+                best = o;
+                pick = p;
             }
         }
-        if (pick < 0) break;
-        const int c = ch[pick];
-        ch[pick] = a.child[c].x;
-        ch[nch++] = a.child[c].y;
+        if (best < 0.0) break;
+        const int c = __shfl_sync(gm, ch, lead + pick);
+        if (sub == pick || sub == nch)
+        {
+            const int2 cc = a.child[c];
+            ch = sub == pick ? cc.x : cc.y;
+            cnt = node_count(ch, n, a.range);
+            cb = a.box[ch];
+            area = cnt > kMaxLeaf ? box_area(cb) : -1.0;
+        }
+        ++nch;
     }
-    Box6 nb;
+    const bool real = sub < nch;
+    float lo[3], hi[3];
     for (int k = 0; k < 3; ++k)
     {
-        nb.lo[k] = FLT_MAX;
-        nb.hi[k] = -FLT_MAX;
-    }
-    for (int i = 0; i < nch; ++i)
-        for (int k = 0; k < 3; ++k)
+        lo[k] = real ? cb.lo[k] : FLT_MAX;
+        hi[k] = real ? cb.hi[k] : -FLT_MAX;
+        for (int j = 4; j > 0; j >>= 1)
         {
-            nb.lo[k] = fminf(nb.lo[k], a.box[ch[i]].lo[k]);
-            nb.hi[k] = fmaxf(nb.hi[k], a.box[ch[i]].hi[k]);
+            lo[k] = fminf(lo[k], __shfl_xor_sync(gm, lo[k], j));
+            hi[k] = fmaxf(hi[k], __shfl_xor_sync(gm, hi[k], j));
         }
-    double nc[3];
-    for (int k = 0; k < 3; ++k) nc[k] = 0.5 * ((double)nb.lo[k] + nb.hi[k]);
+    }
     // octant slots: greedy over (child, slot) by decreasing alignment, ties to
     // the earlier candidate (the host builder's stable sort)
-    double cost[8][8];
-    for (int i = 0; i < nch; ++i)
-    {
-        double off[3];
-        for (int k = 0; k < 3; ++k) off[k] = 0.5 * ((double)a.box[ch[i]].lo[k] + a.box[ch[i]].hi[k]) - nc[k];
-        for (int s = 0; s < 8; ++s)
-        {
-            double c = 0.0;
-            for (int k = 0; k < 3; ++k) c += ((s >> k) & 1) ? off[k] : -off[k];
-            cost[i][s] = c;
-        }
-    }
-    int slot_of[8], child_in_slot[8];
-    for (int i = 0; i < 8; ++i)
-    {
-        slot_of[i] = -1;
-        child_in_slot[i] = -1;
-    }
+    double off[3];
+    for (int k = 0; k < 3; ++k)
+        off[k] = 0.5 * ((double)cb.lo[k] + cb.hi[k]) - 0.5 * ((double)lo[k] + hi[k]);
+    unsigned taken = 0u;
+    int slot = -1;
     for (int round = 0; round < nch; ++round)
     {
-        int bi = -1, bs = -1;
-        double bc = 0.0;
-        for (int i = 0; i < nch; ++i)
-        {
-            if (slot_of[i] >= 0) continue;
+        double bc = -DBL_MAX;
+        int bs = 8;
+        if (real && slot < 0)
             for (int s = 0; s < 8; ++s)
             {
-                if (child_in_slot[s] >= 0) continue;
-                if (bi < 0 || cost[i][s] > bc)
+                if ((taken >> s) & 1u) continue;
+                double c = 0.0;
+                for (int k = 0; k < 3; ++k) c += ((s >> k) & 1) ? off[k] : -off[k];
+                if (bs == 8 || c > bc)
                 {
-                    bc = cost[i][s];
-                    bi = i;
+                    bc = c;
                     bs = s;
                 }
             }
-        }
-        slot_of[bi] = bs;
-        child_in_slot[bs] = bi;
-    }
-    ar_wide_node node;
-    memset(&node, 0, sizeof(node));
-    memset(node.qlo, 0xff, sizeof(node.qlo));  // empty slots: an inverted box that no ray meets
-    node.px = nb.lo[0];
-    node.py = nb.lo[1];
-    node.pz = nb.lo[2];
-    double scale[3];
-    for (int k = 0; k < 3; ++k)
-    {
-        const double ext = (double)nb.hi[k] - nb.lo[k];
-        int e = -126;
-        if (ext > 0.0)
+        int who = bs < 8 ? sub : 8 + sub;
+        for (int k = 4; k > 0; k >>= 1)
         {
-            e = (int)ceil(log2(ext / 255.0));
-            while (ldexp(255.0, e) < ext) ++e;
-            e = max(-126, min(127, e));
+            const double o = __shfl_xor_sync(gm, bc, k);
+            const int w = __shfl_xor_sync(gm, who, k);
+            const int s = __shfl_xor_sync(gm, bs, k);
+            if (w < 8 && (who >= 8 || o > bc || (o == bc && w < who)))
+            {
+                bc = o;
+                who = w;
+                bs = s;
+            }
         }
-        node.e[k] = (uint8_t)(e + 127);
-        scale[k] = ldexp(1.0, e);
+        taken |= 1u << bs;
+        if (sub == who) slot = bs;
     }
-    int n_int = 0, n_prims = 0;
-    for (int i = 0; i < nch; ++i)
-    {
-        const int c = node_count(ch[i], n, a.range);
-        if (c <= kMaxLeaf) n_prims += c;
-        else ++n_int;
-    }
-    const int child_base = n_int ? atomicAdd(a.node_counter, n_int) : 0;
-    const int prim_base = n_prims ? atomicAdd(a.slot_counter, n_prims) : 0;
-    if (child_base + n_int > a.node_cap || prim_base + n_prims > n)
-    {
-        atomicOr(err, AR_DEVERR_QUEUE);
-        return;
-    }
-    node.child_base = (uint32_t)child_base;
-    node.prim_base = (uint32_t)prim_base;
-    const double p[3] = {nb.lo[0], nb.lo[1], nb.lo[2]};
-    int rank = 0, off = 0;
+    // from here lane k holds the child of slot k (or none)
+    int from = -1;
     for (int s = 0; s < 8; ++s)
     {
-        const int ci = child_in_slot[s];
-        if (ci < 0) continue;
-        const int c = ch[ci];
-        const Box6& cb = a.box[c];
-        for (int k = 0; k < 3; ++k)
+        const unsigned m = __ballot_sync(gm, real && slot == s);
+        if (s == sub && m) from = __ffs((int)m) - 1;
+    }
+    const bool used = from >= 0;
+    const int src = used ? from : lane;
+    ch = __shfl_sync(gm, ch, src);
+    cnt = __shfl_sync(gm, cnt, src);
+    for (int k = 0; k < 3; ++k)
+    {
+        cb.lo[k] = __shfl_sync(gm, cb.lo[k], src);
+        cb.hi[k] = __shfl_sync(gm, cb.hi[k], src);
+    }
+    const bool inner = used && cnt > kMaxLeaf, leaf = used && !inner;
+    const unsigned imask = (__ballot_sync(gm, inner) >> lead) & 0xffu;
+    const int n_int = __popc(imask), rank = __popc(imask & ((1u << sub) - 1u));
+    int poff = leaf ? cnt : 0;  // exclusive sum of the leaves' primitives over the slots
+    for (int k = 1; k < 8; k <<= 1)
+    {
+        const int o = __shfl_up_sync(gm, poff, k, 8);
+        if (sub >= k) poff += o;
+    }
+    const int n_prims = __shfl_sync(gm, poff, lead + 7);
+    poff -= leaf ? cnt : 0;
+    int child_base = 0, prim_base = 0, q0 = 0;
+    if (sub == 0)
+    {
+        if (n_int)
         {
-            double ql = floor(((double)cb.lo[k] - p[k]) / scale[k]);
-            double qh = ceil(((double)cb.hi[k] - p[k]) / scale[k]);
-            ql = fmin(fmax(ql, 0.0), 255.0);
-            qh = fmin(fmax(qh, 0.0), 255.0);
-            node.qlo[k][s] = (uint8_t)ql;
-            node.qhi[k][s] = (uint8_t)qh;
+            child_base = atomicAdd(a.node_counter, n_int);
+            q0 = atomicAdd(next_count, n_int);
         }
-        const int cnt = node_count(c, n, a.range);
-        if (cnt > kMaxLeaf)
+        if (n_prims) prim_base = atomicAdd(a.slot_counter, n_prims);
+    }
+    child_base = __shfl_sync(gm, child_base, lead);
+    prim_base = __shfl_sync(gm, prim_base, lead);
+    q0 = __shfl_sync(gm, q0, lead);
+    if (child_base + n_int > a.node_cap || prim_base + n_prims > n || q0 + n_int > a.node_cap)
+    {
+        if (sub == 0) atomicOr(err, AR_DEVERR_QUEUE);
+        return;
+    }
+    ar_wide_node* node = &a.nodes[wi];
+    const uint8_t meta = inner ? (uint8_t)(0x80u | (uint32_t)rank) : leaf ? (uint8_t)(((uint32_t)cnt << 5) | (uint32_t)poff) : 0;
+    node->meta[sub] = meta;
+    int e[3];
+    for (int k = 0; k < 3; ++k)
+    {
+        e[k] = quant_exponent(lo[k], hi[k]);
+        const float inv = ldexpf(1.0f, -e[k]);
+        // empty slots: an inverted box that no ray meets
+        node->qlo[k][sub] = used ? quant_low(cb.lo[k], lo[k], inv) : 0xff;
+        node->qhi[k][sub] = used ? quant_high(cb.hi[k], lo[k], inv) : 0;
+    }
+    if (sub == 0)
+    {
+        node->px = lo[0];
+        node->py = lo[1];
+        node->pz = lo[2];
+        for (int k = 0; k < 3; ++k) node->e[k] = (uint8_t)(e[k] + 127);
+        node->imask = (uint8_t)imask;
+        node->child_base = (uint32_t)child_base;
+        node->prim_base = (uint32_t)prim_base;
+    }
+    if (inner) next[q0 + rank] = make_int2(child_base + rank, ch);
+    if (leaf)
+    {
+        const int first = node_first(ch, n, a.range);
+        for (int j = 0; j < cnt; ++j)
         {
-            node.imask |= (uint8_t)(1u << s);
-            node.meta[s] = (uint8_t)(0x80u | (uint32_t)rank);
-            const int qn = atomicAdd(next_count, 1);
-            if (qn < a.node_cap) next[qn] = make_int2(child_base + rank, c);
-            else atomicOr(err, AR_DEVERR_QUEUE);
-            ++rank;
-        }
-        else
-        {
-            node.meta[s] = (uint8_t)(((uint32_t)cnt << 5) | (uint32_t)off);
-            const int first = node_first(c, n, a.range);
-            for (int j = 0; j < cnt; ++j)
-            {
-                const arbvh::PrimInput& pi = a.prims[a.order[first + j]];
-                ar_prim_slot sl;
-                memset(&sl, 0, sizeof(sl));
-                const uint32_t tag = pi.id | (pi.kind << AR_PRIM_KIND_SHIFT);
-                if (pi.kind == AR_PRIM_KIND_TRI)
-                    for (int k = 0; k < 3; ++k)
-                    {
-                        sl.a[k] = pi.v[k];
-                        sl.b[k] = pi.v[3 + k];
-                        sl.c[k] = pi.v[6 + k];
-                    }
-                sl.a[3] = __uint_as_float(tag);
-                a.slots[prim_base + off + j] = sl;
-            }
-            off += cnt;
+            const arbvh::PrimInput& pi = a.prims[a.order[first + j]];
+            ar_prim_slot sl;
+            memset(&sl, 0, sizeof(sl));
+            const uint32_t tag = pi.id | (pi.kind << AR_PRIM_KIND_SHIFT);
+            if (pi.kind == AR_PRIM_KIND_TRI)
+                for (int k = 0; k < 3; ++k)
+                {
+                    sl.a[k] = pi.v[k];
+                    sl.b[k] = pi.v[3 + k];
+                    sl.c[k] = pi.v[6 + k];
+                }
+            sl.a[3] = __uint_as_float(tag);
+            a.slots[prim_base + poff + j] = sl;
         }
     }
-    a.nodes[wi] = node;
 }
 } // namespace lbvh
 
@@ -520,94 +566,83 @@ __global__ void k_refit_slots(float4* slots, int nslots, const float* __restrict
     }
 }
 
-// one depth of wide nodes: child boxes from the leaves' primitives or the
-// deeper level's node boxes, then the node re-quantized as the builders do
-__global__ void k_refit_level(ar_wide_node* nodes, const int* __restrict__ list, int nlist,
-                              const float4* __restrict__ slots, const float* __restrict__ prim_box, float* node_box)
+// One depth of wide nodes, 8 lanes per node and one per child: child boxes from
+// the leaves' primitives or the deeper level's node boxes, then the node
+// re-quantized as the builders do.  A level near the root has few nodes and costs
+// the chain of one of them: by a single thread (8 children in turn, divisions and
+// logarithms in double precision) 40-60 us, by a group 5 (all 7 levels of a
+// 524,000-triangle sheet: 389 -> 39 us).
+__global__ void __launch_bounds__(128) k_refit_level(ar_wide_node* nodes, const int* __restrict__ list, int nlist,
+                                                   const float4* __restrict__ slots, const float* __restrict__ prim_box,
+                                                   float* node_box)
 {
-    const int li = blockIdx.x * blockDim.x + threadIdx.x;
-    if (li >= nlist) return;
+    const int lane = threadIdx.x & 31, sub = lane & 7, lead = lane & 24;
+    const unsigned gm = 0xffu << lead;
+    const int li = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    if (li >= nlist) return;  // whole groups
     const int ni = list[li];
-    ar_wide_node node = nodes[ni];
-    float cb[8][6];
-    float nb[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-    int rank = 0;
-    for (int s = 0; s < 8; ++s)
+    ar_wide_node* node = &nodes[ni];
+    const uint32_t meta = node->meta[sub], child_base = node->child_base, prim_base = node->prim_base;
+    const unsigned inner = (__ballot_sync(gm, (meta & 0x80u) != 0u) >> lead) & 0xffu;
+    float b[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
+    if (meta & 0x80u)
     {
-        const uint32_t meta = node.meta[s];
-        if (meta == 0u) continue;
-        float b[6] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX};
-        if (meta & 0x80u)
+        const float* src = node_box + 6 * (size_t)(child_base + __popc(inner & ((1u << sub) - 1u)));
+        for (int k = 0; k < 6; ++k) b[k] = src[k];
+    }
+    else if (meta)
+    {
+        const int cnt = (int)(meta >> 5), first = (int)(prim_base + (meta & 31u));
+        for (int j = 0; j < cnt; ++j)
         {
-            const float* src = node_box + 6 * (size_t)(node.child_base + rank);
-            for (int k = 0; k < 6; ++k) b[k] = src[k];
-            ++rank;
-        }
-        else
-        {
-            const int cnt = (int)(meta >> 5), first = (int)(node.prim_base + (meta & 31u));
-            for (int j = 0; j < cnt; ++j)
+            const float4 a = slots[3 * (size_t)(first + j)];
+            const uint32_t tag = __float_as_uint(a.w);
+            if ((tag >> AR_PRIM_KIND_SHIFT) == AR_PRIM_KIND_TRI)
             {
-                const float4 a = slots[3 * (size_t)(first + j)];
-                const uint32_t tag = __float_as_uint(a.w);
-                if ((tag >> AR_PRIM_KIND_SHIFT) == AR_PRIM_KIND_TRI)
+                const float4 bb = slots[3 * (size_t)(first + j) + 1], cc = slots[3 * (size_t)(first + j) + 2];
+                b[0] = fminf(b[0], fminf(a.x, fminf(bb.x, cc.x)));
+                b[1] = fminf(b[1], fminf(a.y, fminf(bb.y, cc.y)));
+                b[2] = fminf(b[2], fminf(a.z, fminf(bb.z, cc.z)));
+                b[3] = fmaxf(b[3], fmaxf(a.x, fmaxf(bb.x, cc.x)));
+                b[4] = fmaxf(b[4], fmaxf(a.y, fmaxf(bb.y, cc.y)));
+                b[5] = fmaxf(b[5], fmaxf(a.z, fmaxf(bb.z, cc.z)));
+            }
+            else
+            {
+                const float* pb = prim_box + 6 * (size_t)(tag & AR_PRIM_ID_MASK);
+                for (int k = 0; k < 3; ++k)
                 {
-                    const float4 bb = slots[3 * (size_t)(first + j) + 1], cc = slots[3 * (size_t)(first + j) + 2];
-                    b[0] = fminf(b[0], fminf(a.x, fminf(bb.x, cc.x)));
-                    b[1] = fminf(b[1], fminf(a.y, fminf(bb.y, cc.y)));
-                    b[2] = fminf(b[2], fminf(a.z, fminf(bb.z, cc.z)));
-                    b[3] = fmaxf(b[3], fmaxf(a.x, fmaxf(bb.x, cc.x)));
-                    b[4] = fmaxf(b[4], fmaxf(a.y, fmaxf(bb.y, cc.y)));
-                    b[5] = fmaxf(b[5], fmaxf(a.z, fmaxf(bb.z, cc.z)));
-                }
-                else
-                {
-                    const float* pb = prim_box + 6 * (size_t)(tag & AR_PRIM_ID_MASK);
-                    for (int k = 0; k < 3; ++k)
-                    {
-                        b[k] = fminf(b[k], pb[k]);
-                        b[3 + k] = fmaxf(b[3 + k], pb[3 + k]);
-                    }
+                    b[k] = fminf(b[k], pb[k]);
+                    b[3 + k] = fmaxf(b[3 + k], pb[3 + k]);
                 }
             }
         }
-        for (int k = 0; k < 6; ++k) cb[s][k] = b[k];
-        for (int k = 0; k < 3; ++k)
-        {
-            nb[k] = fminf(nb[k], b[k]);
-            nb[3 + k] = fmaxf(nb[3 + k], b[3 + k]);
-        }
     }
-    node.px = nb[0];
-    node.py = nb[1];
-    node.pz = nb[2];
-    double scale[3];
     for (int k = 0; k < 3; ++k)
     {
-        const double ext = (double)nb[3 + k] - nb[k];
-        int e = -126;
-        if (ext > 0.0)
+        float lo = b[k], hi = b[3 + k];
+        for (int j = 4; j > 0; j >>= 1)
         {
-            e = (int)ceil(log2(ext / 255.0));
-            while (ldexp(255.0, e) < ext) ++e;
-            e = max(-126, min(127, e));
+            lo = fminf(lo, __shfl_xor_sync(gm, lo, j));
+            hi = fmaxf(hi, __shfl_xor_sync(gm, hi, j));
         }
-        node.e[k] = (uint8_t)(e + 127);
-        scale[k] = ldexp(1.0, e);
-    }
-    for (int s = 0; s < 8; ++s)
-    {
-        if (node.meta[s] == 0u) continue;
-        for (int k = 0; k < 3; ++k)
+        const int e = lbvh::quant_exponent(lo, hi);
+        const float inv = ldexpf(1.0f, -e);
+        if (meta)
         {
-            double ql = floor(((double)cb[s][k] - nb[k]) / scale[k]);
-            double qh = ceil(((double)cb[s][3 + k] - nb[k]) / scale[k]);
-            node.qlo[k][s] = (uint8_t)fmin(fmax(ql, 0.0), 255.0);
-            node.qhi[k][s] = (uint8_t)fmin(fmax(qh, 0.0), 255.0);
+            node->qlo[k][sub] = lbvh::quant_low(b[k], lo, inv);
+            node->qhi[k][sub] = lbvh::quant_high(b[3 + k], lo, inv);
+        }
+        if (sub == 0)
+        {
+            if (k == 0) node->px = lo;
+            else if (k == 1) node->py = lo;
+            else node->pz = lo;
+            node->e[k] = (uint8_t)(e + 127);
+            node_box[6 * (size_t)ni + k] = lo;
+            node_box[6 * (size_t)ni + 3 + k] = hi;
         }
     }
-    nodes[ni] = node;
-    for (int k = 0; k < 6; ++k) node_box[6 * (size_t)ni + k] = nb[k];
 }
 
 cudaError_t refit_wide_bvh(Ctx& c, const float* verts_dev, cudaStream_t s)
@@ -621,7 +656,7 @@ cudaError_t refit_wide_bvh(Ctx& c, const float* verts_dev, cudaStream_t s)
     {
         const int a = c.refit_level_off[d], b = c.refit_level_off[d + 1];
         if (b <= a) continue;
-        k_refit_level<<<(b - a + 127) / 128, 128, 0, s>>>(reinterpret_cast<ar_wide_node*>(c.d_nodes), c.d_refit_nodes + a,
+        k_refit_level<<<(b - a + 15) / 16, 128, 0, s>>>(reinterpret_cast<ar_wide_node*>(c.d_nodes), c.d_refit_nodes + a,
                                                          b - a, reinterpret_cast<const float4*>(c.d_slots), c.d_prim_box,
                                                          c.d_node_box);
         e = cudaGetLastError();
@@ -722,7 +757,7 @@ std::string build_wide_bvh_gpu(const std::vector<arbvh::PrimInput>& prims, arbvh
         ++depth;
         e = cudaMemsetAsync(&counters[2], 0, sizeof(int), s);
         if (e != cudaSuccess) break;
-        k_collapse<<<(nq + 127) / 128, 128, 0, s>>>(ca, qa, nq, qb, &counters[2], (unsigned int*)&counters[3]);
+        k_collapse<<<(nq + 15) / 16, 128, 0, s>>>(ca, qa, nq, qb, &counters[2], (unsigned int*)&counters[3]);
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaMemcpyAsync(&nq, &counters[2], sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
