@@ -308,15 +308,9 @@ __global__ void __launch_bounds__(AR_BLOCK) k_raygen(PathState ps, int* queue, i
 #ifndef AR_SHD_REFILL_MIN0
 #define AR_SHD_REFILL_MIN0 16    // shadow rays of the first vertices (16: 6.55 ms of the same render, 32: 6.75)
 #endif
-#ifndef AR_SHADE_MLP_MIN_BLOCKS
-#define AR_SHADE_MLP_MIN_BLOCKS 2    // k_shade<2> (MLP guide): blocks per SM it is compiled for (at 1,
-                                     // 201 registers and 11 % of warps active: 3.5 % slower)
-#endif
-#ifndef AR_SHADE_PATHS_PER_THREAD
-#define AR_SHADE_PATHS_PER_THREAD 16  // k_shade's grid: one thread per this many paths of the wave (a
-                                      // grid-stride loop that prefetches each next pass's path state;
-                                      // 64-spp terrain step: 2, 4, 8, 16 paths per thread gave 85.1,
-                                      // 83.8, 83.0, 82.8 ms)
+#ifndef AR_PASS_PATHS
+#define AR_PASS_PATHS 16         // grid of the passes over a whole queue (k_partition, the guide query and the
+                                 // analytic SDF objects): one thread per this many paths of the wave
 #endif
 #ifndef AR_TRAV_MIN_BLOCKS
 #define AR_TRAV_MIN_BLOCKS 4     // blocks per SM the traversal kernels are compiled for (64 registers)
@@ -804,12 +798,6 @@ __global__ void __launch_bounds__(AR_BLOCK) k_mlp_query(DevScene sc, PathState p
 }
 
 // ---------------------------------------------------------------- shade
-#ifndef AR_SHADE_LEAN_MIN_BLOCKS
-#define AR_SHADE_LEAN_MIN_BLOCKS 2  // the same for the opaque-surface instantiation (AR_FEAT_SURFACE)
-#endif
-#ifndef AR_SHADE_MIN_BLOCKS
-#define AR_SHADE_MIN_BLOCKS 2    // blocks per SM the unguided / voxel-guided shade kernels are compiled for
-#endif
 struct ShadeParams
 {
     int use_nee;
@@ -946,13 +934,17 @@ __global__ void __launch_bounds__(AR_BLOCK) k_partition(const int* __restrict__ 
 
 // Scene features a k_shade instantiation handles, fixed at compile time: the
 // BSDF models (AR_MATS_* bits), the participating medium and albedo textures.
-// Scenes of opaque surfaces only (no glass, medium or textures, the camera
-// outside every object) run an instantiation without that code: the same
-// arithmetic for everything it keeps, less code and fewer registers.
+// Scenes of opaque surfaces only (no glass or medium, the camera outside every
+// object) run an instantiation without that code, with or without textures: the
+// same arithmetic for everything it keeps, less code and fewer registers
+// (textured Cornell box 256 x 256, forward and replay: 24.8 ms with every
+// feature compiled in, 22.8 without glass and medium; voxel guide 480 x 270
+// untextured 8.9 ms with every feature, 8.2 with AR_FEAT_SURFACE).
 #define AR_FEAT_MEDIUM (1 << 4)
 #define AR_FEAT_TEX (1 << 5)
 #define AR_FEAT_ALL (AR_MATS_ALL | AR_FEAT_MEDIUM | AR_FEAT_TEX)
 #define AR_FEAT_SURFACE (AR_MATS_DIFFUSE | AR_MATS_LIGHT | AR_MATS_GGX)
+#define AR_FEAT_TEXTURED (AR_FEAT_SURFACE | AR_FEAT_TEX)
 
 // The shadow ray a vertex casts for its light sample, and what it adds to the
 // path's radiance either way.
@@ -1000,8 +992,12 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
     h.nrm = v3(0, 0, 0);
     h.local_pos = v3(0, 0, 0);
     BsdfSample S = bsdf_sample_default();
-    Material mat;
-    mat.shading = AR_MAT_DIFFUSE;
+    // the hit's material: read where it is used (a copy would stay in registers
+    // through the whole vertex); a textured one is a copy with its texel's colour
+    constexpr bool TEX = (FEAT & AR_FEAT_TEX) != 0;
+    const Material* mp = sc.materials;
+    Material textured;
+#define VERTEX_MAT (TEX ? textured : *mp)
     if (active)
     {
         const float4 ro = ps.ray_o[p], rd = ps.ray_d[p];
@@ -1070,18 +1066,22 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
         }
         if (h.hit)
         {
-            mat = sc.materials[h.material];
-            if ((FEAT & AR_FEAT_TEX) && mat.albedo_tex >= 0 && sc.tex_count > 0)
+            mp = sc.materials + h.material;
+            if constexpr (TEX)
             {
-                texel = albedo_texel(sc, mat.albedo_tex, slot, h.obj, h.pos);
-                if (texel >= 0)
+                textured = *mp;
+                if (textured.albedo_tex >= 0 && sc.tex_count > 0)
                 {
-                    const float* tx = sc.texels + 3 * (size_t)texel;
-                    mat.albedo = v3(__ldg(tx), __ldg(tx + 1), __ldg(tx + 2));
-                    mat.albedo_c = prepare_color(mat.albedo, PlainFetch{sc.lut_rgb});
+                    texel = albedo_texel(sc, textured.albedo_tex, slot, h.obj, h.pos);
+                    if (texel >= 0)
+                    {
+                        const float* tx = sc.texels + 3 * (size_t)texel;
+                        textured.albedo = v3(__ldg(tx), __ldg(tx + 1), __ldg(tx + 2));
+                        textured.albedo_c = prepare_color(textured.albedo, PlainFetch{sc.lut_rgb});
+                    }
                 }
             }
-            S = evaluate_material<FEAT & AR_MATS_ALL>(lambda, lb, R, mat, rayD, h, media);
+            S = evaluate_material<FEAT & AR_MATS_ALL>(lambda, lb, R, VERTEX_MAT, rayD, h, media);
         }
         else if (scatter)
         {
@@ -1113,7 +1113,7 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
             if (prm.gbuf && depth == 0)
             {
                 const int mid = h.hit ? h.material : -1;
-                const V3 alb = h.hit ? mat.albedo : v3(0.0f, 0.0f, 0.0f);
+                const V3 alb = h.hit ? VERTEX_MAT.albedo : v3(0.0f, 0.0f, 0.0f);
                 prm.gbuf[2 * (size_t)p] = make_float4(alb.x, alb.y, alb.z, __int_as_float(mid));
                 prm.gbuf[2 * (size_t)p + 1] = make_float4(h.nrm.x, h.nrm.y, h.nrm.z, h.dist);
             }
@@ -1157,9 +1157,9 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
                             const GuideSample g = mlp_sample_hemisphere(q, q_total, R, h.nrm);
                             if (dot(g.dir, h.nrm) > 1.0e-12f)
                             {
-                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
+                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, VERTEX_MAT, h.nrm, rayD, g.dir);
                                 S.next_dir = g.dir;
-                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
+                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, VERTEX_MAT, rayD, g.dir, h, media);
                                 S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
                             }
                             else
@@ -1194,9 +1194,9 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
                             const GuideSample g = sample_octahedron_hemisphere(*probe, R, h.nrm, maskq);
                             if (dot(g.dir, h.nrm) > 1.0e-12f)
                             {
-                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, g.dir);
+                                const float pBs = bsdf_pdf<FEAT & AR_MATS_ALL>(lb, VERTEX_MAT, h.nrm, rayD, g.dir);
                                 S.next_dir = g.dir;
-                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, g.dir, h, media);
+                                S.brdf = eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, VERTEX_MAT, rayD, g.dir, h, media);
                                 S.pdf = (1.0f - pgProb) * fmaxf(pBs, 1.0e-12f) + pgProb * g.pdf;
                             }
                             else
@@ -1249,7 +1249,7 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
                 if (pL >= 0.0f && pB > 0.0f) misW = power_heuristic(pB, pL);
             }
             endpointLe = S.emissive * misW;
-            radiance = radiance + mask * interact(mat.emissive_c, lb) * d65 * misW;
+            radiance = radiance + mask * interact(VERTEX_MAT.emissive_c, lb) * d65 * misW;
         }
         else if (!all_zero(S.emissive))
         {
@@ -1271,14 +1271,14 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
                 g_med_albedo -= dlt * mask * sc.medium.emission * d65;
                 g_med_emission += dlt * medium_unit;
             }
-            if (prm.grad && texel >= 0 && mat.shading == AR_MAT_DIFFUSE)
+            if (prm.grad && texel >= 0 && VERTEX_MAT.shading == AR_MAT_DIFFUSE)
             {
                 const float rest = ps.adj_total[p] - radiance;
                 const float dlt = ps.adj_delta[p];
-                const float alb = interact(mat.albedo_c, lb);
+                const float alb = interact(VERTEX_MAT.albedo_c, lb);
                 if (rest != 0.0f && dlt != 0.0f && alb > 1.0e-8f)
                 {
-                    const V3 g = interact_rgb_grad(lb, mat.albedo, PlainFetch{sc.lut_rgb}) * (dlt * rest / alb);
+                    const V3 g = interact_rgb_grad(lb, VERTEX_MAT.albedo, PlainFetch{sc.lut_rgb}) * (dlt * rest / alb);
                     float* gp = prm.grad + 3 * (size_t)texel;
                     if (g.x != 0.0f) atomicAdd(gp + 0, g.x);
                     if (g.y != 0.0f) atomicAdd(gp + 1, g.y);
@@ -1356,13 +1356,13 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
                         {
                             const float brdfCos =
                                 scatter ? sc.medium.albedo * hg_pdf(dot(rayD, L), sc.medium.g)
-                                        : eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, mat, rayD, L, h, media_default());
+                                        : eval_bsdf_cos<FEAT & AR_MATS_ALL>(lambda, lb, VERTEX_MAT, rayD, L, h, media_default());
                             const float G = (cosY / dist2);
                             const float le = interact(sc.materials[ls.material].emissive_c, lb);
                             const float contribution = brdfCos * le * (G / pATotal);
                             const float pLight = area_to_solid_angle_pdf(h.pos, ls.point, ls.normal, ls.p_facet * ls.p_a);
                             float pBsdf = scatter ? hg_pdf(dot(rayD, L), sc.medium.g)
-                                                  : fmaxf(bsdf_pdf<FEAT & AR_MATS_ALL>(lb, mat, h.nrm, rayD, L), 0.0f);
+                                                  : fmaxf(bsdf_pdf<FEAT & AR_MATS_ALL>(lb, VERTEX_MAT, h.nrm, rayD, L), 0.0f);
                             if constexpr (GUIDE)
                             {
                                 if (probe)
@@ -1467,6 +1467,8 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
     return keep;
 }
 
+#undef VERTEX_MAT
+
 // the wavelength LUT into shared memory
 __device__ __forceinline__ void stage_lambda_lut(const DevScene& sc, float* s_lam)
 {
@@ -1490,8 +1492,8 @@ __device__ __forceinline__ void add_medium_gradient(double* grad_medium, float g
 }
 
 // What bounds k_shade is instruction supply: one vertex runs some 2,800
-// instructions of mostly straight-line code (45 KB), the SM holds 16 warps
-// (128 registers), and when each warp is somewhere else in that code most
+// instructions of mostly straight-line code (45 KB), the SM holds 16 to 28 warps
+// (128 to 72 registers), and when each warp is somewhere else in that code most
 // stalls are instruction fetches (256x256x16 Cornell box: 3.7 of 10.4 warps per
 // issue; voxel guide: 14.0 of 21.5).  A barrier at the top of each pass and one
 // before next-event estimation keep a block's warps in the same part of the
@@ -1500,10 +1502,23 @@ __device__ __forceinline__ void add_medium_gradient(double* grad_medium, float g
 // voxel guide 480x270x16 6.23 -> 4.29 ms.  The opaque-surface instantiation
 // keeps only the first one: its waves on large scenes wait for memory
 // (1920x1080x32 terrain 9.83 ms with one barrier, 10.04 with both, 9.89 with
-// none).  More barriers, or blocks of 512, gain nothing further.
+// none).  More barriers gain nothing further.
+//
+// Threads per block, two blocks on an SM: shading waits on instruction fetch and
+// on scattered loads, so the leaner instantiations, which spill little at fewer
+// registers, do better with more warps. Measured on the stage's time: opaque
+// untextured (1080p terrain) 10.0 ms at 256 threads, 9.2 at 320, 8.8 at 384, 8.9 at
+// 448; the same with the voxel guide (480 x 270) 3.75 ms at 256, 3.5 at 320, 3.6 at
+// 384, 3.3 at 448. The others keep 256: textured 256 x 256 with its replay 22.8 ms
+// for a whole step, 23.1 at 320, 23.7 at 384, and the full set of materials spills
+// at 128 registers already.
+template <int GUIDE, bool ADJ, int FEAT>
+constexpr int kShadeBlock = FEAT != AR_FEAT_SURFACE ? 256 : GUIDE ? 448 : 384;
+constexpr int AR_SHADE_RESIDENT = 2;  // blocks on an SM
+constexpr int AR_SHADE_PASSES = 8;    // paths per thread before the grid grows; 4 to 32 measure alike
+
 template <int GUIDE, bool ADJ, int FEAT = AR_FEAT_ALL>
-__global__ void __launch_bounds__(AR_BLOCK, GUIDE == 2 ? AR_SHADE_MLP_MIN_BLOCKS
-                                            : (FEAT == AR_FEAT_SURFACE ? AR_SHADE_LEAN_MIN_BLOCKS : AR_SHADE_MIN_BLOCKS))
+__global__ void __launch_bounds__((kShadeBlock<GUIDE, ADJ, FEAT>), AR_SHADE_RESIDENT)
     k_shade(DevScene sc, PathState ps, ShadowQueue sq, const int2* __restrict__ queue,
                                                   const int* __restrict__ counter, int* next_queue, int* next_counter,
                                                   int* shadow_counter, ShadeParams prm)
@@ -1944,6 +1959,32 @@ static void launch_sdf_shadow(const DevScene& sc, const PathState& ps, const Sha
     if (sc.trav.sdf.count > 0) k_sdf_shadow<<<grid_m, AR_BLOCK, 0, s>>>(sc.trav.sdf, ps, sq, pend, &cnt[AR_CNT_SDF + 1]);
 }
 
+struct ShadeArgs
+{
+    const DevScene& sc;
+    const PathState& ps;
+    const ShadowQueue& sq;
+    const int2* queue;
+    const int* counter;
+    int* next_queue;
+    int* next_counter;
+    int* shadow_counter;
+    const ShadeParams& prm;
+    long long bound;  // paths at most
+    int sms;
+    cudaStream_t stream;
+};
+
+template <int GUIDE, bool ADJ, int FEAT>
+static void launch_shade(const ShadeArgs& a)
+{
+    constexpr int B = kShadeBlock<GUIDE, ADJ, FEAT>;
+    const long long resident = (long long)AR_SHADE_RESIDENT * a.sms;
+    const int grid = (int)(resident * std::max<long long>(1, a.bound / (resident * B * AR_SHADE_PASSES)));
+    k_shade<GUIDE, ADJ, FEAT><<<grid, B, 0, a.stream>>>(a.sc, a.ps, a.sq, a.queue, a.counter, a.next_queue, a.next_counter,
+                                                        a.shadow_counter, a.prm);
+}
+
 // records a stage interval when profiling
 struct StageScope
 {
@@ -1985,14 +2026,18 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     const int grid_t = sms * AR_TRAV_MIN_BLOCKS, grid_m = sms * AR_SDF_MIN_BLOCKS;
     int* cnt = c.d_counters;  // AR_CNT_* layout
     const CamParams cam = make_camera(rl);
-    // opaque surfaces only: the shading instantiation without glass, medium and texture code
-    bool lean = !c.medium.on && c.tex_count == 0 && !c.camera_inside && !rl.guide && !rl.adjoint;
-    for (const Material& m : c.materials) lean = lean && m.shading != AR_MAT_GLASS;
+    // SDF geometry: its work leaves the traversal kernels for k_sdf_extend / k_sdf_shadow
+    const bool has_sdf = c.sdf_object_count > 0 || c.sdf.count > 0;
+    // opaque surfaces only: the shading instantiations without glass and medium
+    // code (and without textures, where the scene has none); the MLP guide has one only
+    bool opaque_tex = !c.medium.on && !c.camera_inside && rl.guide != 2;
+    for (const Material& m : c.materials) opaque_tex = opaque_tex && m.shading != AR_MAT_GLASS;
+    const bool opaque = opaque_tex && c.tex_count == 0;
     {
         StageScope st(c, ST_RAYGEN);
         k_raygen<<<grid_n, AR_BLOCK, 0, s>>>(c.ps, c.d_queue[0], &cnt[AR_CNT_Q0], first_path, n, rl.width, rl.height,
-                                             rl.seed, rl.first_frame, cam, c.camera_inside, &cnt[AR_CNT_FETCH], !lean,
-                                             rl.guide != 0, path_order(rl), rl.jumps);
+                                             rl.seed, rl.first_frame, cam, c.camera_inside, &cnt[AR_CNT_FETCH],
+                                             !opaque || has_sdf || rl.adjoint, rl.guide != 0, path_order(rl), rl.jumps);
         if (rl.guide) k_guide_init<<<grid_n, AR_BLOCK, 0, s>>>(c.ps, n);
     }
     long long L = rl.guide ? 2 : 1;
@@ -2007,8 +2052,6 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     net.wbf = c.d_mlp_wbf;
     net.w32 = c.d_mlp_w32;
     net.box = c.mlp_box;
-    // SDF geometry: its work leaves the traversal kernels for k_sdf_extend / k_sdf_shadow
-    const bool has_sdf = c.sdf_object_count > 0 || c.sdf.count > 0;
     const int n_sdf = (sc.sdf_trav.node_count > 0 ? 1 : 0) + (sc.trav.sdf.count > 0 ? 1 : 0);  // launches of each pass
     const SdfPending pend_shd{has_sdf ? c.d_pend_list : nullptr, &cnt[AR_CNT_PEND]};
     // Each depth's next-queue length is copied to pinned host memory behind
@@ -2045,14 +2088,14 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
             const int* fn = &cnt[AR_CNT_Q0 + (b & 1)];
             const auto finish = has_sdf ? (rl.adjoint ? k_finish<true, AR_FEAT_ALL, true> : k_finish<false, AR_FEAT_ALL, true>)
                                 : rl.adjoint ? k_finish<true, AR_FEAT_ALL, false>
-                                : lean       ? k_finish<false, AR_FEAT_SURFACE, false>
+                                : opaque     ? k_finish<false, AR_FEAT_SURFACE, false>
                                              : k_finish<false, AR_FEAT_ALL, false>;
             finish<<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
             ++L;
             break;
         }
-        const int grid_s = std::max(2 * sms, (int)((bound + AR_BLOCK * AR_SHADE_PATHS_PER_THREAD - 1) /
-                                                   (AR_BLOCK * AR_SHADE_PATHS_PER_THREAD)));
+        const int grid_s = std::max(2 * sms, (int)((bound + AR_BLOCK * AR_PASS_PATHS - 1) /
+                                                   (AR_BLOCK * AR_PASS_PATHS)));
         const int cur = b & 1, nxt = cur ^ 1;
         int* qn = &cnt[AR_CNT_Q0 + cur];
         // k_extend zeroes the next queue, shadow queue, shadow fetch and pending
@@ -2089,16 +2132,13 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
             int* nq = c.d_queue[nxt];
             int* nn = &cnt[AR_CNT_Q0 + nxt];
             const int2* pq = c.d_pq;
-            if (rl.guide == 2)
-                k_shade<2, false><<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm);
-            else if (rl.guide)
-                k_shade<1, false><<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm);
-            else if (rl.adjoint)
-                k_shade<0, true><<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm);
-            else if (lean)
-                k_shade<0, false, AR_FEAT_SURFACE><<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm);
-            else
-                k_shade<0, false><<<grid_s, AR_BLOCK, 0, s>>>(sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm);
+            const ShadeArgs sa{sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm, bound, sms, s};
+            if (rl.guide == 2) launch_shade<2, false, AR_FEAT_ALL>(sa);
+            else if (rl.guide) opaque ? launch_shade<1, false, AR_FEAT_SURFACE>(sa) : launch_shade<1, false, AR_FEAT_ALL>(sa);
+            else if (rl.adjoint) opaque_tex ? launch_shade<0, true, AR_FEAT_TEXTURED>(sa) : launch_shade<0, true, AR_FEAT_ALL>(sa);
+            else if (opaque) launch_shade<0, false, AR_FEAT_SURFACE>(sa);
+            else if (opaque_tex) launch_shade<0, false, AR_FEAT_TEXTURED>(sa);
+            else launch_shade<0, false, AR_FEAT_ALL>(sa);
         }
         {
             StageScope st(c, ST_SHADOW);
@@ -2146,7 +2186,7 @@ cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int grid_n = (n + AR_BLOCK - 1) / AR_BLOCK;
     const int grid_t = sms * AR_TRAV_MIN_BLOCKS, grid_m = sms * AR_SDF_MIN_BLOCKS;
-    const int grid_s = std::max(2 * sms, (n + AR_BLOCK * AR_SHADE_PATHS_PER_THREAD - 1) / (AR_BLOCK * AR_SHADE_PATHS_PER_THREAD));
+    const int grid_s = std::max(2 * sms, (n + AR_BLOCK * AR_PASS_PATHS - 1) / (AR_BLOCK * AR_PASS_PATHS));
     int* cnt = wb.counters;  // AR_CNT_* layout
     const CamParams cam = make_camera(rl);
     k_raygen<<<grid_n, AR_BLOCK, 0, s>>>(wb.ps, wb.queue[0], &cnt[AR_CNT_Q0], first_path, n, rl.width, rl.height, rl.seed,
@@ -2174,8 +2214,8 @@ cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb
             launch_sdf_extend(sc, wb.ps, wb.queue[cur], &cnt[AR_CNT_Q0 + cur], cnt, grid_s, grid_m, s);
         k_partition<<<grid_s, AR_BLOCK, 0, s>>>(wb.queue[cur], wb.ps.q_slot, &cnt[AR_CNT_Q0 + cur], wb.pq,
                                                 &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1]);
-        k_shade<0, false><<<grid_s, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, wb.pq, &cnt[AR_CNT_Q0 + cur],
-                                                   wb.queue[nxt], &cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], prm);
+        launch_shade<0, false, AR_FEAT_ALL>(ShadeArgs{sc, wb.ps, wb.sq, wb.pq, &cnt[AR_CNT_Q0 + cur], wb.queue[nxt],
+                                                      &cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], prm, n, sms, s});
         k_shadow<<<grid_t, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, &cnt[AR_CNT_SHADOW], &cnt[AR_CNT_FETCH + 1], pend_shd, err,
                                              b == 0 ? AR_SHD_REFILL_MIN0 : AR_SHD_REFILL_MIN, shd_rs);
         if (has_sdf) launch_sdf_shadow(sc, wb.ps, wb.sq, pend_shd, cnt, grid_s, grid_m, s);
