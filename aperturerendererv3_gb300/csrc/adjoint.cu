@@ -1,24 +1,33 @@
 // Replay adjoint of the albedo textures (no counterpart in the reference).
 //
-// ar_adjoint runs every wave twice over the same random streams: the first
-// pass is the ordinary render and leaves each path's total radiance L; the
-// seed kernel below turns d(loss)/d(image) into the path's scalar adjoint
-// delta = sum_c dl/dXYZ_c * dXYZ_c/dL / spp; the second pass (k_shade<*, true>)
-// scatters delta * (L - radiance so far) * d(albedo)/d(rgb) / albedo into a
-// float32 gradient buffer at every textured diffuse vertex.  After each wave
-// the float32 buffer is folded into the caller's float64 gradient and
-// cleared, so float32 sums only ever span one wave.
+// ar_adjoint renders every wave once, with shading (k_shade<0, AR_ADJ_RECORD, *>)
+// leaving per vertex the texel whose colour it used and the radiance of the path
+// so far.  k_adjoint_scatter then knows each path's total radiance L, turns
+// d(loss)/d(image) into the path's scalar adjoint
+// delta = sum_c dl/dXYZ_c * dXYZ_c/dL / spp and adds
+// delta * (L - radiance so far) * d(albedo)/d(rgb) / albedo into a float32
+// gradient buffer for every textured diffuse vertex.  After each wave the
+// float32 buffer is folded into the caller's float64 gradient and cleared, so
+// float32 sums only ever span one wave.
+//
+// Depth limits whose records would pass AR_ADJ_RECORDS_MAX, and the medium's
+// parameters (ar_adjoint_medium), render every wave twice over the same random
+// streams instead: an ordinary pass for L, k_adjoint_seed for delta, and a
+// replay (k_shade<0, AR_ADJ_REPLAY, *>) that scatters as it goes.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 
 #include "ar_internal.h"
 
 namespace ar
 {
-__global__ void k_adjoint_seed(DevScene sc, PathState ps, int n, const float* __restrict__ dl_dxyz, float inv_spp)
+#define AR_SCATTER_BLOCK 256
+
+// A path's total radiance and d(loss)/d(radiance).
+__device__ __forceinline__ float2 path_adjoint(const DevScene& sc, const PathState& ps, int k, float lambda,
+                                               const float* __restrict__ dl_dxyz, float inv_spp)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const float lambda = ps.ray_o[k].w;
     const float pdf = ps.ray_d[k].w;
     float r = ps.radiance[k];
     if (!(r == r) || fabsf(r) == __int_as_float(0x7f800000)) r = 0.0f;
@@ -31,8 +40,51 @@ __global__ void k_adjoint_seed(DevScene sc, PathState ps, int n, const float* __
     if (cx > 0.0f && cx < AR_RADIANCE_CLAMP) d += g[0] * (xyz.x / pdf);
     if (cy > 0.0f && cy < AR_RADIANCE_CLAMP) d += g[1] * (xyz.y / pdf);
     if (cz > 0.0f && cz < AR_RADIANCE_CLAMP) d += g[2] * (xyz.z / pdf);
-    ps.adj_total[k] = r;
-    ps.adj_delta[k] = d * inv_spp;
+    return make_float2(r, d * inv_spp);
+}
+
+__global__ void k_adjoint_seed(DevScene sc, PathState ps, int n, const float* __restrict__ dl_dxyz, float inv_spp)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const float2 a = path_adjoint(sc, ps, k, ps.ray_o[k].w, dl_dxyz, inv_spp);
+    ps.adj_total[k] = a.x;
+    ps.adj_delta[k] = a.y;
+}
+
+__global__ void __launch_bounds__(AR_SCATTER_BLOCK)
+    k_adjoint_scatter(DevScene sc, PathState ps, int n, int max_depth, const float* __restrict__ dl_dxyz, float inv_spp,
+                      float* __restrict__ grad)
+{
+    __shared__ float s_lam[AR_LAMBDA_LUT_RES * 4];
+    for (int i = threadIdx.x; i < AR_LAMBDA_LUT_RES * 4; i += blockDim.x) s_lam[i] = sc.lut_lambda[i];
+    __syncthreads();
+    const int stride = gridDim.x * blockDim.x;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride)
+    {
+        const float lambda = ps.ray_o[k].w;
+        const float2 a = path_adjoint(sc, ps, k, lambda, dl_dxyz, inv_spp);
+        if (a.y == 0.0f) continue;
+        const Basis lb = query_lambda(lambda, s_lam);
+        const PlainFetch f{sc.lut_rgb};
+        // the state keeps the depth of the path's last vertex
+        const int vertices = min((int)(ps.depths[k] & 0xffffu) + 1, max_depth);
+        for (int v = 0; v < vertices; ++v)
+        {
+            const int2 rec = ps.adj_rec[(size_t)v * ps.adj_stride + k];
+            const float rest = a.x - __int_as_float(rec.y);
+            if (rec.x < 0 || rest == 0.0f) continue;
+            const float* tx = sc.texels + 3 * (size_t)rec.x;
+            const V3 rgb = v3(__ldg(tx), __ldg(tx + 1), __ldg(tx + 2));
+            const float alb = interact(prepare_color(rgb, f), lb);
+            if (!(alb > 1.0e-8f)) continue;
+            const V3 g = interact_rgb_grad(lb, rgb, f) * (a.y * rest / alb);
+            float* gp = grad + 3 * (size_t)rec.x;
+            if (g.x != 0.0f) atomicAdd(gp + 0, g.x);
+            if (g.y != 0.0f) atomicAdd(gp + 1, g.y);
+            if (g.z != 0.0f) atomicAdd(gp + 2, g.z);
+        }
+    }
 }
 
 __global__ void k_grad_fold(float* __restrict__ g32, double* __restrict__ g64, long long n)
@@ -53,6 +105,19 @@ cudaError_t launch_adjoint_seed(Ctx& c, const RenderLaunch& rl, int n, const flo
 {
     const DevScene sc = dev_scene(c);
     k_adjoint_seed<<<(n + 255) / 256, 256, 0, c.stream>>>(sc, c.ps, n, dl_dxyz, 1.0f / (float)rl.spp);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_scatter(Ctx& c, const RenderLaunch& rl, int n, const float* dl_dxyz, float* grad,
+                                   long long* launches)
+{
+    const DevScene sc = dev_scene(c);
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    const int grid = std::min((n + AR_SCATTER_BLOCK - 1) / AR_SCATTER_BLOCK, sms * 8);
+    k_adjoint_scatter<<<grid, AR_SCATTER_BLOCK, 0, c.stream>>>(sc, c.ps, n, rl.max_depth, dl_dxyz, 1.0f / (float)rl.spp,
+                                                               grad);
     if (launches) *launches += 1;
     return cudaGetLastError();
 }

@@ -19,6 +19,12 @@ namespace ar
 #define AR_WAVE_PATHS_AUTO (1 << 25)      // ar_render's automatic wave size
 #define AR_BOUNCE_LOOKAHEAD 4             // depths the host queues ahead of the queue lengths it has read
 #define AR_WAVE_PATHS_ADJOINT (1 << 21)   // ar_adjoint's
+#define AR_ADJ_REPLAY 1                   // RenderLaunch::adjoint: scatter gradients while replaying the paths
+#define AR_ADJ_RECORD 2                   // leave a record per vertex for k_adjoint_scatter
+// ar_adjoint records a wave's vertices when its paths times the depth limit stay
+// within this many records (1 GiB), and replays the wave otherwise.  The default
+// wave holds 64 depths.
+#define AR_ADJ_RECORDS_MAX (1ll << 27)
 
 // Order of a frame's pixels among the paths of a wave: bands of 4 rows, each
 // cut into chunks 8 pixels wide taken left to right, row by row inside a
@@ -271,10 +277,13 @@ struct PathState
     float4* pg_dir;     // xyz sampled direction, w = collected radiance
     float4* pg_loc;     // xyz vertex position, w = radiance mask
     float4* pg_vdir;    // xyz reflected direction (voxel face key)
-    // replay adjoint only: the path's total radiance (first pass) and
-    // d(loss)/d(radiance)
+    // adjoint only: the path's total radiance and d(loss)/d(radiance) for the
+    // replay pass; per depth and path {texel or -1, bits(radiance before the
+    // vertex)} for the recording pass
     float* adj_total;
     float* adj_delta;
+    int2* adj_rec;
+    int adj_stride;     // paths per depth of adj_rec
     // MLP guide only: network inputs of the path's current hit and the 64
     // quantised cell weights inferred for it
     float4* q_pos;      // xyz hit position, w = 1 when the query is valid
@@ -302,7 +311,7 @@ struct RenderLaunch
     int first_frame;
     int profile;
     int guide;    // 0 none, 1 voxel probes, 2 MLP (voxel probes until the network has trained)
-    int adjoint;  // 1: replay pass of ar_adjoint (gradient scatter, no output)
+    int adjoint;  // pass of ar_adjoint (AR_ADJ_*, no output), or 0
     float* grad;  // replay pass: float32 texel gradients
     int mlp_ready;  // guide 2: sample from the network instead of the voxel probes
     double* grad_medium;  // replay pass of ar_adjoint_medium: d loss / d (albedo, emission)
@@ -397,6 +406,8 @@ struct Ctx
     long long grad32_n = 0;
     float* d_adj = nullptr;              // 2 floats per wave path
     int adj_capacity = 0;
+    int2* d_adj_rec = nullptr;           // recording pass: one record per depth and path of a wave
+    size_t adj_rec_n = 0;
     double* d_grad_medium = nullptr;     // d loss / d (medium albedo, medium emission)
     // smooth-union SDF object and the participating medium
     std::vector<float> sdf_prims;        // 8 floats per primitive
@@ -523,10 +534,12 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
                                float* per_sample_out, long long* launches);
 cudaError_t launch_accumulate(Ctx& c, const RenderLaunch& rl, long long first_path, int n_paths, double* accum,
                               long long* launches);
-// replay adjoint (adjoint.cu): per-path seed between the two passes, and the
-// float32 -> float64 gradient fold after each wave
+// adjoint (adjoint.cu): per-path seed before the replay pass, or the scatter of a
+// recorded wave; the float32 -> float64 gradient fold after each wave
 cudaError_t launch_adjoint_seed(Ctx& c, const RenderLaunch& rl, int n_paths, const float* dl_dxyz,
                                 long long* launches);
+cudaError_t launch_adjoint_scatter(Ctx& c, const RenderLaunch& rl, int n_paths, const float* dl_dxyz, float* grad,
+                                   long long* launches);
 cudaError_t launch_grad_fold(Ctx& c, double* grad64, long long n, long long* launches);
 // denoiser (denoise.cu): fold one wave's first-hit records and sample XYZ into
 // the per-pixel records, in sample order

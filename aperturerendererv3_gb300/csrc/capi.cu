@@ -742,6 +742,7 @@ ar_status ar_destroy(ar_ctx* ctx)
     free_dev(c.d_stats);
     free_dev(c.d_grad32);
     free_dev(c.d_adj);
+    free_dev(c.d_adj_rec);
     free_dev(c.d_grad_medium);
     free_dev(c.d_frame_xyz);
     free_dev(c.d_frame_dn);
@@ -1426,9 +1427,10 @@ ar_status ar_render(ar_ctx* ctx, const ar_render_params* prm, double* out_xyz, i
 
 namespace
 {
-// Replay adjoint driver: per wave a radiance pass, the per-path seed and the
-// replay pass that scatters gradients (texels into float32, folded into
-// grad_texels in float64 after each wave; medium parameters into grad_medium).
+// Adjoint driver.  Texel gradients: per wave a recording pass and the scatter of
+// its records into float32, folded into grad_texels in float64 after each wave;
+// waves with too many records, and the medium's parameters (into grad_medium),
+// take a radiance pass, the per-path seed and a replay pass instead.
 ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_dxyz, double* grad_texels,
                       double* grad_medium, void* stream)
 {
@@ -1446,14 +1448,29 @@ ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_
     if ((long long)cap > total) cap = (int)total;
     st = ensure_waves(ctx, cap);
     if (st != AR_OK) return st;
-    if (c.adj_capacity < c.ps.capacity)
+    const long long records = (long long)cap * rl.max_depth;
+    bool record = grad_texels && records <= AR_ADJ_RECORDS_MAX;
+    if (record && c.adj_rec_n < (size_t)records)
+    {
+        free_dev(c.d_adj_rec);
+        c.adj_rec_n = 0;
+        if (alloc_dev(c.d_adj_rec, (size_t)records) == cudaSuccess) c.adj_rec_n = (size_t)records;
+        else
+        {
+            cudaGetLastError();  // no room for the records: replay
+            record = false;
+        }
+    }
+    c.ps.adj_rec = c.d_adj_rec;
+    c.ps.adj_stride = cap;
+    if (!record && c.adj_capacity < c.ps.capacity)
     {
         free_dev(c.d_adj);
         AR_CUDA(ctx, alloc_dev(c.d_adj, 2 * (size_t)c.ps.capacity));
         c.adj_capacity = c.ps.capacity;
     }
     c.ps.adj_total = c.d_adj;
-    c.ps.adj_delta = c.d_adj + c.ps.capacity;
+    c.ps.adj_delta = c.d_adj ? c.d_adj + c.ps.capacity : nullptr;
     if (grad_texels)
     {
         if (c.grad32_n < c.texel_floats)
@@ -1472,16 +1489,24 @@ ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_
     cudaEventRecord(e0, c.stream);
     long long launches = 0;
     cudaError_t e = cudaSuccess;
-    RenderLaunch replay = rl;
-    replay.adjoint = 1;
-    replay.grad = grad_texels ? c.d_grad32 : nullptr;
-    replay.grad_medium = grad_medium;
+    RenderLaunch pass = rl;  // the recording or the replay pass
+    pass.adjoint = record ? AR_ADJ_RECORD : AR_ADJ_REPLAY;
+    pass.grad = grad_texels ? c.d_grad32 : nullptr;
+    pass.grad_medium = grad_medium;
     for (long long first = 0; first < total && e == cudaSuccess;)
     {
         const int n = (int)std::min<long long>(cap, total - first);
-        e = launch_render_wave(c, rl, first, n, nullptr, &launches);                           // radiance of each path
-        if (e == cudaSuccess) e = launch_adjoint_seed(c, rl, n, dl_dxyz, &launches);           // its adjoint
-        if (e == cudaSuccess) e = launch_render_wave(c, replay, first, n, nullptr, &launches);  // replay + scatter
+        if (record)
+        {
+            e = launch_render_wave(c, pass, first, n, nullptr, &launches);
+            if (e == cudaSuccess) e = launch_adjoint_scatter(c, rl, n, dl_dxyz, c.d_grad32, &launches);
+        }
+        else
+        {
+            e = launch_render_wave(c, rl, first, n, nullptr, &launches);                          // radiance of each path
+            if (e == cudaSuccess) e = launch_adjoint_seed(c, rl, n, dl_dxyz, &launches);          // its adjoint
+            if (e == cudaSuccess) e = launch_render_wave(c, pass, first, n, nullptr, &launches);  // replay + scatter
+        }
         if (e == cudaSuccess && grad_texels) e = launch_grad_fold(c, grad_texels, c.texel_floats, &launches);
         first += n;
     }
@@ -1493,6 +1518,7 @@ ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_
     c.last_launches = launches;
     c.ps.adj_total = nullptr;
     c.ps.adj_delta = nullptr;
+    c.ps.adj_rec = nullptr;
     c.profile = 0;
     if (e != cudaSuccess) return cuda_fail(ctx, e, "adjoint");
     unsigned int word = 0;

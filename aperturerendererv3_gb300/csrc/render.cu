@@ -964,13 +964,13 @@ struct ShadowRay
 // Without glass the path never enters an object: its media record stays
 // the default and is neither read nor written.  Unguided forward renders
 // read nothing of an ended path but its radiance.
-template <int GUIDE, bool ADJ, int FEAT, bool SYNC_NEE>
+template <int GUIDE, int ADJ, int FEAT, bool SYNC_NEE>
 __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState& ps, const ShadeParams& prm,
                                              const float* s_lam, bool active, int p, int slot, int2 next, ShadowRay& sh,
                                              float& g_med_albedo, float& g_med_emission)
 {
     constexpr bool TRACK_MEDIA = (FEAT & AR_MATS_GLASS) != 0;
-    constexpr bool STORE_ENDED = GUIDE != 0 || ADJ;
+    constexpr bool STORE_ENDED = GUIDE != 0 || ADJ == AR_ADJ_REPLAY;
     bool keep = false;
     // state of the vertex, across the phases below
     V3 rayO = v3(0, 0, 0), rayD = v3(0, 0, 0);
@@ -1255,7 +1255,13 @@ __device__ __forceinline__ bool shade_vertex(const DevScene& sc, const PathState
         {
             endpointLe = S.emissive;
         }
-        if constexpr (ADJ)
+        if constexpr (ADJ == AR_ADJ_RECORD)
+        {
+            // what the gradient of this vertex's texel needs once the path's total is known
+            const bool albedo_hit = texel >= 0 && VERTEX_MAT.shading == AR_MAT_DIFFUSE;
+            ps.adj_rec[(size_t)depth * ps.adj_stride + p] = make_int2(albedo_hit ? texel : -1, __float_as_int(radiance));
+        }
+        if constexpr (ADJ == AR_ADJ_REPLAY)
         {
             // replay adjoint: every contribution still to come on this path
             // (NEE here, emission and NEE further on) carries this vertex's
@@ -1512,12 +1518,12 @@ __device__ __forceinline__ void add_medium_gradient(double* grad_medium, float g
 // 384, 3.3 at 448. The others keep 256: textured 256 x 256 with its replay 22.8 ms
 // for a whole step, 23.1 at 320, 23.7 at 384, and the full set of materials spills
 // at 128 registers already.
-template <int GUIDE, bool ADJ, int FEAT>
+template <int GUIDE, int ADJ, int FEAT>
 constexpr int kShadeBlock = FEAT != AR_FEAT_SURFACE ? 256 : GUIDE ? 448 : 384;
 constexpr int AR_SHADE_RESIDENT = 2;  // blocks on an SM
 constexpr int AR_SHADE_PASSES = 8;    // paths per thread before the grid grows; 4 to 32 measure alike
 
-template <int GUIDE, bool ADJ, int FEAT = AR_FEAT_ALL>
+template <int GUIDE, int ADJ, int FEAT = AR_FEAT_ALL>
 __global__ void __launch_bounds__((kShadeBlock<GUIDE, ADJ, FEAT>), AR_SHADE_RESIDENT)
     k_shade(DevScene sc, PathState ps, ShadowQueue sq, const int2* __restrict__ queue,
                                                   const int* __restrict__ counter, int* next_queue, int* next_counter,
@@ -1559,7 +1565,7 @@ __global__ void __launch_bounds__((kShadeBlock<GUIDE, ADJ, FEAT>), AR_SHADE_RESI
             sq.sdf_eps[sqi] = sh.sdf_eps;
         }
     }
-    if constexpr (ADJ)
+    if constexpr (ADJ == AR_ADJ_REPLAY)
     {
         if (prm.grad_medium) add_medium_gradient(prm.grad_medium, g_med_albedo, g_med_emission);
     }
@@ -1782,7 +1788,7 @@ __device__ __forceinline__ bool shadow_path(const DevScene& sc, const ShadowRay&
 
 // Every queued path to its end: the arithmetic of k_extend, k_shade and k_shadow
 // per path, in the same order.
-template <bool ADJ, int FEAT, bool SDF>
+template <int ADJ, int FEAT, bool SDF>
 __global__ void __launch_bounds__(AR_FINISH_BLOCK, AR_FINISH_MIN_BLOCKS)
     k_finish(DevScene sc, PathState ps, const int* __restrict__ queue, const int* __restrict__ counter, ShadeParams prm,
              unsigned int* err)
@@ -1812,7 +1818,7 @@ __global__ void __launch_bounds__(AR_FINISH_BLOCK, AR_FINISH_MIN_BLOCKS)
             active = keep;
         }
     }
-    if constexpr (ADJ)
+    if constexpr (ADJ == AR_ADJ_REPLAY)
     {
         if (prm.grad_medium) add_medium_gradient(prm.grad_medium, g_med_albedo, g_med_emission);
     }
@@ -1975,7 +1981,7 @@ struct ShadeArgs
     cudaStream_t stream;
 };
 
-template <int GUIDE, bool ADJ, int FEAT>
+template <int GUIDE, int ADJ, int FEAT>
 static void launch_shade(const ShadeArgs& a)
 {
     constexpr int B = kShadeBlock<GUIDE, ADJ, FEAT>;
@@ -2086,10 +2092,14 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
                                                         (long long)sms * AR_FINISH_MIN_BLOCKS);
             const int* fq = c.d_queue[b & 1];
             const int* fn = &cnt[AR_CNT_Q0 + (b & 1)];
-            const auto finish = has_sdf ? (rl.adjoint ? k_finish<true, AR_FEAT_ALL, true> : k_finish<false, AR_FEAT_ALL, true>)
-                                : rl.adjoint ? k_finish<true, AR_FEAT_ALL, false>
-                                : opaque     ? k_finish<false, AR_FEAT_SURFACE, false>
-                                             : k_finish<false, AR_FEAT_ALL, false>;
+            const bool replay = rl.adjoint == AR_ADJ_REPLAY;
+            const auto finish = rl.adjoint && has_sdf ? (replay ? k_finish<AR_ADJ_REPLAY, AR_FEAT_ALL, true>
+                                                                : k_finish<AR_ADJ_RECORD, AR_FEAT_ALL, true>)
+                                : rl.adjoint          ? (replay ? k_finish<AR_ADJ_REPLAY, AR_FEAT_ALL, false>
+                                                                : k_finish<AR_ADJ_RECORD, AR_FEAT_ALL, false>)
+                                : has_sdf             ? k_finish<0, AR_FEAT_ALL, true>
+                                : opaque              ? k_finish<0, AR_FEAT_SURFACE, false>
+                                                      : k_finish<0, AR_FEAT_ALL, false>;
             finish<<<grid_f, AR_FINISH_BLOCK, 0, s>>>(sc, c.ps, fq, fn, prm, c.d_err);
             ++L;
             break;
@@ -2133,12 +2143,14 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
             int* nn = &cnt[AR_CNT_Q0 + nxt];
             const int2* pq = c.d_pq;
             const ShadeArgs sa{sc, c.ps, c.sq, pq, qn, nq, nn, shc, prm, bound, sms, s};
-            if (rl.guide == 2) launch_shade<2, false, AR_FEAT_ALL>(sa);
-            else if (rl.guide) opaque ? launch_shade<1, false, AR_FEAT_SURFACE>(sa) : launch_shade<1, false, AR_FEAT_ALL>(sa);
-            else if (rl.adjoint) opaque_tex ? launch_shade<0, true, AR_FEAT_TEXTURED>(sa) : launch_shade<0, true, AR_FEAT_ALL>(sa);
-            else if (opaque) launch_shade<0, false, AR_FEAT_SURFACE>(sa);
-            else if (opaque_tex) launch_shade<0, false, AR_FEAT_TEXTURED>(sa);
-            else launch_shade<0, false, AR_FEAT_ALL>(sa);
+            if (rl.guide == 2) launch_shade<2, 0, AR_FEAT_ALL>(sa);
+            else if (rl.guide) opaque ? launch_shade<1, 0, AR_FEAT_SURFACE>(sa) : launch_shade<1, 0, AR_FEAT_ALL>(sa);
+            else if (rl.adjoint == AR_ADJ_REPLAY) launch_shade<0, AR_ADJ_REPLAY, AR_FEAT_ALL>(sa);
+            else if (rl.adjoint)
+                opaque_tex ? launch_shade<0, AR_ADJ_RECORD, AR_FEAT_TEXTURED>(sa) : launch_shade<0, AR_ADJ_RECORD, AR_FEAT_ALL>(sa);
+            else if (opaque) launch_shade<0, 0, AR_FEAT_SURFACE>(sa);
+            else if (opaque_tex) launch_shade<0, 0, AR_FEAT_TEXTURED>(sa);
+            else launch_shade<0, 0, AR_FEAT_ALL>(sa);
         }
         {
             StageScope st(c, ST_SHADOW);
@@ -2214,7 +2226,7 @@ cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb
             launch_sdf_extend(sc, wb.ps, wb.queue[cur], &cnt[AR_CNT_Q0 + cur], cnt, grid_s, grid_m, s);
         k_partition<<<grid_s, AR_BLOCK, 0, s>>>(wb.queue[cur], wb.ps.q_slot, &cnt[AR_CNT_Q0 + cur], wb.pq,
                                                 &cnt[AR_CNT_PART], &cnt[AR_CNT_PART + 1]);
-        launch_shade<0, false, AR_FEAT_ALL>(ShadeArgs{sc, wb.ps, wb.sq, wb.pq, &cnt[AR_CNT_Q0 + cur], wb.queue[nxt],
+        launch_shade<0, 0, AR_FEAT_ALL>(ShadeArgs{sc, wb.ps, wb.sq, wb.pq, &cnt[AR_CNT_Q0 + cur], wb.queue[nxt],
                                                       &cnt[AR_CNT_Q0 + nxt], &cnt[AR_CNT_SHADOW], prm, n, sms, s});
         k_shadow<<<grid_t, AR_BLOCK, 0, s>>>(sc, wb.ps, wb.sq, &cnt[AR_CNT_SHADOW], &cnt[AR_CNT_FETCH + 1], pend_shd, err,
                                              b == 0 ? AR_SHD_REFILL_MIN0 : AR_SHD_REFILL_MIN, shd_rs);
