@@ -23,6 +23,7 @@
 namespace ar
 {
 #define AR_SCATTER_BLOCK 256
+#define AR_SCATTER_MIN_BLOCKS 4
 
 // A path's total radiance and d(loss)/d(radiance).
 __device__ __forceinline__ float2 path_adjoint(const DevScene& sc, const PathState& ps, int k, float lambda,
@@ -52,7 +53,14 @@ __global__ void k_adjoint_seed(DevScene sc, PathState ps, int n, const float* __
     ps.adj_delta[k] = a.y;
 }
 
-__global__ void __launch_bounds__(AR_SCATTER_BLOCK)
+// One thread per path, over its records.  Bound by the gathers from the spectral
+// table (eight corners of 16 bytes per record, each its own sector: the texels
+// of a texture name cells all over the 2 GB) and by the atomics; 4.2 million
+// paths of depth 8 over 512 x 512 textures took 2.45 ms with the corners read as
+// 4-byte loads.  With 16-byte loads the whole 256 x 256 x 64 step takes 16.3 ms at
+// 4 blocks per SM (64 registers), 16.6 / 16.5 / 17.4 at 5 / 6 / 8, and 16.7 with
+// one thread per record, which repeats the path's part for each.
+__global__ void __launch_bounds__(AR_SCATTER_BLOCK, AR_SCATTER_MIN_BLOCKS)
     k_adjoint_scatter(DevScene sc, PathState ps, int n, int max_depth, const float* __restrict__ dl_dxyz, float inv_spp,
                       float* __restrict__ grad)
 {
@@ -115,7 +123,7 @@ cudaError_t launch_adjoint_scatter(Ctx& c, const RenderLaunch& rl, int n, const 
     const DevScene sc = dev_scene(c);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    const int grid = std::min((n + AR_SCATTER_BLOCK - 1) / AR_SCATTER_BLOCK, sms * 8);
+    const int grid = std::min((n + AR_SCATTER_BLOCK - 1) / AR_SCATTER_BLOCK, sms * AR_SCATTER_MIN_BLOCKS * 2);
     k_adjoint_scatter<<<grid, AR_SCATTER_BLOCK, 0, c.stream>>>(sc, c.ps, n, rl.max_depth, dl_dxyz, 1.0f / (float)rl.spp,
                                                                grad);
     if (launches) *launches += 1;

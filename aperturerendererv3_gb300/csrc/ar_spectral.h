@@ -149,13 +149,21 @@ AR_HD Basis query_rgb_basis_f(V3 rgb, const Fetch& fetch)
     return r;
 }
 
+// A voxel's basis: one 16-byte load on the device, where the table is an
+// allocation of its own (four 4-byte loads kept the LSU pipe, not memory, the
+// limit of k_adjoint_scatter).
 struct PlainFetch
 {
     const float* lut;
     AR_HD void operator()(size_t voxel, float* v) const
     {
+#ifdef __CUDA_ARCH__
+        const float4 q = __ldg(reinterpret_cast<const float4*>(lut) + voxel);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+#else
         const float* p = lut + voxel * 4;
         v[0] = p[0]; v[1] = p[1]; v[2] = p[2]; v[3] = p[3];
+#endif
     }
 };
 
