@@ -86,6 +86,12 @@ AR_HD void path_slot(const PathOrder& o, unsigned long long g, uint32_t* u, uint
         const uint32_t fb = g32 / pb;
         const uint32_t r = g32 - fb * pb;
         const uint32_t sb = path_block_samples(o, fb);
+        if (AR_PATH_GROUP_PX == 1u)
+        {
+            *u = r / sb;
+            *s = fb * o.block + (r - *u * sb);
+            return;
+        }
         const uint32_t group = AR_PATH_GROUP_PX * sb;
         const uint32_t ub = r / group;
         const uint32_t w = r - ub * group;
@@ -532,7 +538,9 @@ cudaError_t launch_trace(const DevScene& sc, const float* rays, int n, int any, 
                          unsigned int* err, cudaStream_t s, long long* launches);
 cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_path, int n_paths,
                                float* per_sample_out, long long* launches);
-cudaError_t launch_accumulate(Ctx& c, const RenderLaunch& rl, long long first_path, int n_paths, double* accum,
+// stored: the wave's samples are in out_xyz (launch_render_wave leaves them there for
+// per-sample output and for the denoiser's records only)
+cudaError_t launch_accumulate(Ctx& c, const RenderLaunch& rl, long long first_path, int n_paths, bool stored, double* accum,
                               long long* launches);
 // adjoint (adjoint.cu): per-path seed before the replay pass, or the scatter of a
 // recorded wave; the float32 -> float64 gradient fold after each wave

@@ -1357,7 +1357,7 @@ ar_status ar_render(ar_ctx* ctx, const ar_render_params* prm, double* out_xyz, i
         if (rl.guide) n_ll = std::min<long long>(n_ll, window - first % window);
         const int n = (int)n_ll;
         e = launch_render_wave(c, rl, first, n, d_samples, &launches);
-        if (e == cudaSuccess) e = launch_accumulate(c, rl, first, n, c.d_accum, &launches);
+        if (e == cudaSuccess) e = launch_accumulate(c, rl, first, n, d_samples || rl.denoise, c.d_accum, &launches);
         if (e == cudaSuccess && rl.denoise) e = launch_denoise_record(c, rl, first, n, &launches);
         if (e == cudaSuccess && per_sample_xyz)
             e = cudaMemcpyAsync(per_sample_xyz + 3 * first, d_samples, (size_t)n * 3 * sizeof(float), cudaMemcpyDeviceToHost, c.stream);
