@@ -360,6 +360,7 @@ struct Ctx
     float4* d_sdf_params = nullptr;
     int sdf_object_count = 0;                   // SDF objects in the scene
     int build_mode = 0;                         // AR_BUILD_HOST / AR_BUILD_GPU
+    int node_count = 0, slot_count = 0;         // of the main BVH
     // refit: wide nodes grouped by depth, mesh indices, per-primitive bounds of the rest
     std::vector<int> refit_level_off;           // depth d: nodes [off[d], off[d+1]) of d_refit_nodes
     int* d_refit_nodes = nullptr;
@@ -560,8 +561,27 @@ void free_denoise(Ctx& c);
 void free_volumes(Ctx& c);
 // the smooth union's cell grid (sdfvol.cu), from c.sdf's primitives and bounds
 cudaError_t build_sdf_cells(Ctx& c);
-// GPU BVH build (bvh_gpu.cu): same format as arbvh::build_wide_bvh; "" on success
-std::string build_wide_bvh_gpu(const std::vector<arbvh::PrimInput>& prims, arbvh::WideBVH& out, cudaStream_t s);
+// GPU BVH build (bvh_gpu.cu): same format as arbvh::build_wide_bvh, left on the
+// device.  The primitives are `objects` and then nmesh triangles (9 floats each
+// at mesh_v) with ids from first_mesh_id.  "" on success.
+struct GpuBvh
+{
+    const ar_wide_node* nodes = nullptr;
+    const ar_prim_slot* slots = nullptr;
+    int node_count = 0, slot_count = 0, depth = 0;
+    std::vector<int> level_off;  // depth d: nodes [off[d], off[d + 1])
+    float root_lo[3] = {0, 0, 0}, root_hi[3] = {0, 0, 0};
+    void* arena = nullptr;  // everything above on the device, until the scene has its copies
+    ~GpuBvh() { cudaFree(arena); }
+};
+std::string build_wide_bvh_gpu(const std::vector<arbvh::PrimInput>& objects, const float* mesh_v, int nmesh, int first_mesh_id,
+                               GpuBvh& out, cudaStream_t s);
+// slot tables of a scene (bvh_gpu.cu): prim_slot[id] = slot, and with prim_material
+// the material and light index in the spare lanes of the triangle slots
+cudaError_t launch_slot_tables(void* slots, int n, const int* prim_material, const int* prim_light, int* prim_slot,
+                               cudaStream_t s);
+cudaError_t launch_light_ids(const Light* lights, int n, int* prim_light, cudaStream_t s);
+cudaError_t launch_iota(int* v, int n, cudaStream_t s);
 // refit of the main BVH after mesh vertices moved (bvh_gpu.cu)
 cudaError_t refit_wide_bvh(Ctx& c, const float* verts_dev, cudaStream_t s);
 } // namespace ar

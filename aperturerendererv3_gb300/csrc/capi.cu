@@ -36,7 +36,7 @@ DevScene dev_scene(const Ctx& c)
     s.trav.sdf_vols = c.d_vols;
     s.trav.sdf_vol_count = (int)c.vol_dev.size();
 
-    s.trav.node_count = (int)c.bvh.nodes.size();
+    s.trav.node_count = c.node_count;
     s.materials = c.d_materials;
     s.prim_material = c.d_prim_material;
     s.prim_light = c.d_prim_light;
@@ -950,8 +950,13 @@ ar_status ar_scene_build(ar_ctx* ctx)
     if ((long long)nobj + nmesh == 0) return fail(ctx, AR_ERR_INVALID, "scene has no object or triangle besides the SDF");
     for (int i = 0; i < nobj; ++i)
         if (c.object_material[i] < 0 || c.object_material[i] >= nmat) return fail(ctx, AR_ERR_INVALID, "object material index out of range");
-    for (int i = 0; i < nmesh; ++i)
-        if (c.mesh_material[i] < 0 || c.mesh_material[i] >= nmat) return fail(ctx, AR_ERR_INVALID, "mesh material index out of range");
+    int mesh_mat_lo = 0, mesh_mat_hi = -1;
+    for (const int m : c.mesh_material)
+    {
+        mesh_mat_lo = std::min(mesh_mat_lo, m);
+        mesh_mat_hi = std::max(mesh_mat_hi, m);
+    }
+    if (mesh_mat_lo < 0 || mesh_mat_hi >= nmat) return fail(ctx, AR_ERR_INVALID, "mesh material index out of range");
     const int ntex = (int)(c.tex_sizes.size() / 2);
     for (int i = 0; i < nmat; ++i)
         if (c.materials[i].albedo_tex >= ntex) return fail(ctx, AR_ERR_INVALID, "material texture index out of range");
@@ -986,32 +991,26 @@ ar_status ar_scene_build(ar_ctx* ctx)
         }
     }
 
-    // primitives for the BVH (the SDF object, if any, is marched after the BVH traversal)
+    // primitives for the BVH (the SDF union, if any, is marched after the BVH
+    // traversal); the GPU build makes the mesh's itself.  SDF objects get their own
+    // BVH, traversed in a separate pass, so the main traversal carries no SDF code
     const long long nbvh = (long long)nobj + nmesh;
-    std::vector<arbvh::PrimInput> prims((size_t)nbvh);
-    std::vector<int> prim_material((size_t)nprim), prim_light((size_t)nprim, -1);
-    if (nsdf) prim_material[nbvh] = c.sdf_material;
-    for (long long i = 0; i < nbvh; ++i)
+    const bool gpu_build = c.build_mode == AR_BUILD_GPU;
+    std::vector<arbvh::PrimInput> prims, sdf_prims;
+    prims.reserve(gpu_build ? (size_t)nobj : (size_t)nbvh);
+    for (long long i = 0; i < (gpu_build ? (long long)nobj : nbvh); ++i)
     {
-        arbvh::PrimInput& p = prims[i];
+        arbvh::PrimInput p{};
         p.id = (uint32_t)i;
         const float* tv = nullptr;
-        if (i < nobj)
-        {
-            prim_material[i] = c.object_material[i];
-            if (c.object_type[i] == AR_OBJECT_TRIANGLE) tv = &c.object_tri[9 * (size_t)i];
-            else
-            {
-                p.kind = c.object_type[i] == AR_OBJECT_CUBE   ? AR_PRIM_KIND_BOX
-                         : c.object_type[i] == AR_OBJECT_SDF ? AR_PRIM_KIND_SDF
-                                                             : AR_PRIM_KIND_SPHERE;
-                object_bounds(c.objects[i], p.lo, p.hi);
-            }
-        }
+        if (i >= nobj) tv = &c.mesh_v[9 * (size_t)(i - nobj)];
+        else if (c.object_type[i] == AR_OBJECT_TRIANGLE) tv = &c.object_tri[9 * (size_t)i];
         else
         {
-            prim_material[i] = c.mesh_material[i - nobj];
-            tv = &c.mesh_v[9 * (size_t)(i - nobj)];
+            p.kind = c.object_type[i] == AR_OBJECT_CUBE   ? AR_PRIM_KIND_BOX
+                     : c.object_type[i] == AR_OBJECT_SDF ? AR_PRIM_KIND_SDF
+                                                         : AR_PRIM_KIND_SPHERE;
+            object_bounds(c.objects[i], p.lo, p.hi);
         }
         if (tv)
         {
@@ -1023,26 +1022,20 @@ ar_status ar_scene_build(ar_ctx* ctx)
                 p.hi[k] = std::max(tv[k], std::max(tv[3 + k], tv[6 + k]));
             }
         }
-    }
-    // SDF objects get their own BVH, traversed in a separate pass, so the main
-    // traversal carries no SDF code
-    std::vector<arbvh::PrimInput> sdf_prims;
-    {
-        size_t w = 0;
-        for (size_t i = 0; i < prims.size(); ++i)
-        {
-            if (prims[i].kind == AR_PRIM_KIND_SDF) sdf_prims.push_back(prims[i]);
-            else prims[w++] = prims[i];
-        }
-        prims.resize(w);
+        (p.kind == AR_PRIM_KIND_SDF ? sdf_prims : prims).push_back(p);
     }
     const int n_sdf_objects = (int)sdf_prims.size();
     std::string err;
+    GpuBvh gpu;
     const auto tb0 = std::chrono::steady_clock::now();
-    if (c.build_mode == AR_BUILD_GPU)
+    c.bvh = arbvh::WideBVH{};
+    if (gpu_build)
     {
-        err = build_wide_bvh_gpu(prims, c.bvh, c.stream);
+        err = build_wide_bvh_gpu(prims, c.mesh_v.data(), nmesh, nobj, gpu, c.stream);
         if (!err.empty()) return fail(ctx, AR_ERR_CUDA, err);
+        c.bvh.depth = gpu.depth;
+        std::copy(gpu.root_lo, gpu.root_lo + 3, c.bvh.root_lo);
+        std::copy(gpu.root_hi, gpu.root_hi + 3, c.bvh.root_hi);
     }
     else if (!arbvh::build_wide_bvh(prims, c.bvh, &err))
         return fail(ctx, AR_ERR_INVALID, "BVH build: " + err);
@@ -1052,32 +1045,26 @@ ar_status ar_scene_build(ar_ctx* ctx)
     if (!sdf_prims.empty() && !arbvh::build_wide_bvh(sdf_prims, c.sdf_bvh, &err))
         return fail(ctx, AR_ERR_INVALID, "SDF object BVH build: " + err);
     if (c.sdf_bvh.depth >= AR_TRAV_STACK) return fail(ctx, AR_ERR_INVALID, "SDF object BVH deeper than the traversal stack");
-    std::vector<int> prim_slot((size_t)nprim, -1);
-    for (const arbvh::WideBVH* b : {&c.bvh, &c.sdf_bvh})
-        for (size_t s = 0; s < b->slots.size(); ++s)
-        {
-            uint32_t tag;
-            std::memcpy(&tag, &b->slots[s].a[3], 4);
-            prim_slot[tag & AR_PRIM_ID_MASK] = (int)s;  // SDF objects: a slot of the SDF objects' BVH
-        }
 
     // light table (core/scene.cu:677-706): every primitive with a light material
     c.lights.clear();
     float total = 0.0f;
     std::vector<float> weights;
-    for (long long i = 0; i < nprim; ++i)
+    bool mesh_light = false;  // whether any mesh triangle can be a light
+    for (int m = 0; m < nmat && nmesh > 0; ++m) mesh_light = mesh_light || c.materials[m].shading == AR_MAT_LIGHT;
+    for (long long i = 0; i < (mesh_light ? nbvh : (long long)nobj); ++i)  // an SDF union is never a light
     {
-        const Material& m = c.materials[prim_material[i]];
+        const int mi = i < nobj ? c.object_material[i] : c.mesh_material[i - nobj];
+        const Material& m = c.materials[mi];
         if (m.shading != AR_MAT_LIGHT) continue;
         Light L;
         L.obj = (int)i;
         L.type = (i < nobj) ? c.object_type[i] : AR_OBJ_TRIANGLE;
-        L.material = prim_material[i];
+        L.material = mi;
         const float area = (i < nobj) ? object_area(c.objects[i]) : 0.0f;
         const float w = fmaxf(area * luminance(m.emissive), 1.0e-20f);
         total += w;
         weights.push_back(w);
-        prim_light[i] = (int)c.lights.size();
         c.lights.push_back(L);
     }
     float acc = 0.0f;
@@ -1095,53 +1082,80 @@ ar_status ar_scene_build(ar_ctx* ctx)
     c.sdf_object_count = n_sdf_objects;
     std::vector<Object> objs(c.objects);
     if (objs.empty()) objs.resize(1);
-    AR_CUDA(ctx, alloc_dev(c.d_nodes, c.bvh.nodes.size() * sizeof(ar_wide_node)));
-    AR_CUDA(ctx, cudaMemcpy(c.d_nodes, c.bvh.nodes.data(), c.bvh.nodes.size() * sizeof(ar_wide_node), cudaMemcpyHostToDevice));
-    // triangle slots carry their primitive's material and light index in the
-    // spare w lanes of their second and third float4 (read by the shading's hit
-    // reconstruction; the traversal reads only the vertices and the tag)
-    for (ar_prim_slot& sl : c.bvh.slots)
+    c.node_count = gpu_build ? gpu.node_count : (int)c.bvh.nodes.size();
+    c.slot_count = gpu_build ? gpu.slot_count : (int)c.bvh.slots.size();
+    // the BVH, on the context's stream like the kernels that finish its tables
+    const size_t node_bytes = (size_t)c.node_count * sizeof(ar_wide_node), slot_bytes = (size_t)c.slot_count * sizeof(ar_prim_slot);
+    AR_CUDA(ctx, alloc_dev(c.d_nodes, node_bytes));
+    AR_CUDA(ctx, alloc_dev(c.d_slots, slot_bytes));
+    if (c.node_count > 0)
     {
-        uint32_t tag;
-        std::memcpy(&tag, &sl.a[3], 4);
-        if ((tag >> AR_PRIM_KIND_SHIFT) != AR_PRIM_KIND_TRI) continue;
-        const int32_t mi = prim_material[tag & AR_PRIM_ID_MASK], li = prim_light[tag & AR_PRIM_ID_MASK];
-        std::memcpy(&sl.b[3], &mi, 4);
-        std::memcpy(&sl.c[3], &li, 4);
+        const cudaMemcpyKind from = gpu_build ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        const void* nodes = gpu_build ? gpu.nodes : c.bvh.nodes.data();
+        const void* slots = gpu_build ? gpu.slots : c.bvh.slots.data();
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_nodes, nodes, node_bytes, from, c.stream));
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_slots, slots, slot_bytes, from, c.stream));
     }
-    AR_CUDA(ctx, alloc_dev(c.d_slots, c.bvh.slots.size() * sizeof(ar_prim_slot)));
-    AR_CUDA(ctx, cudaMemcpy(c.d_slots, c.bvh.slots.data(), c.bvh.slots.size() * sizeof(ar_prim_slot), cudaMemcpyHostToDevice));
-    if (nmesh > 0 && !c.bvh.nodes.empty())
+    // per-primitive tables: material, light index or -1, slot or -1 (SDF objects: a
+    // slot of the SDF objects' BVH).  Triangle slots carry their primitive's material
+    // and light index in the spare w lanes of their second and third float4 (read by
+    // the shading's hit reconstruction; the traversal reads only the vertices and the tag)
+    AR_CUDA(ctx, alloc_dev(c.d_prim_material, (size_t)nprim));
+    if (nobj > 0)
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_prim_material, c.object_material.data(), nobj * sizeof(int), cudaMemcpyHostToDevice, c.stream));
+    if (nmesh > 0)
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_prim_material + nobj, c.mesh_material.data(), nmesh * sizeof(int), cudaMemcpyHostToDevice,
+                                     c.stream));
+    if (nsdf)
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_prim_material + nbvh, &c.sdf_material, sizeof(int), cudaMemcpyHostToDevice, c.stream));
+    AR_CUDA(ctx, alloc_dev(c.d_lights, c.lights.size()));
+    if (!c.lights.empty())
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_lights, c.lights.data(), c.lights.size() * sizeof(Light), cudaMemcpyHostToDevice, c.stream));
+    AR_CUDA(ctx, alloc_dev(c.d_prim_light, (size_t)nprim));
+    AR_CUDA(ctx, cudaMemsetAsync(c.d_prim_light, 0xff, nprim * sizeof(int), c.stream));
+    AR_CUDA(ctx, launch_light_ids(c.d_lights, (int)c.lights.size(), c.d_prim_light, c.stream));
+    AR_CUDA(ctx, alloc_dev(c.d_prim_slot, (size_t)nprim));
+    AR_CUDA(ctx, cudaMemsetAsync(c.d_prim_slot, 0xff, nprim * sizeof(int), c.stream));
+    AR_CUDA(ctx, launch_slot_tables(c.d_slots, c.slot_count, c.d_prim_material, c.d_prim_light, c.d_prim_slot, c.stream));
+    if (nmesh > 0 && c.node_count > 0)
     {
         // refit tables: wide nodes by depth (children always follow their parent), mesh
         // indices, the bounds of the non-triangle primitives
-        std::vector<int> level_nodes, cur{0}, next;
-        c.refit_level_off.assign(1, 0);
-        while (!cur.empty())
+        AR_CUDA(ctx, alloc_dev(c.d_refit_nodes, (size_t)c.node_count));
+        if (gpu_build)
         {
-            next.clear();
-            for (int ni : cur)
+            c.refit_level_off = gpu.level_off;
+            AR_CUDA(ctx, launch_iota(c.d_refit_nodes, c.node_count, c.stream));
+        }
+        else
+        {
+            std::vector<int> level_nodes, cur{0}, next;
+            c.refit_level_off.assign(1, 0);
+            while (!cur.empty())
             {
-                level_nodes.push_back(ni);
-                const ar_wide_node& nd = c.bvh.nodes[ni];
-                int rank = 0;
-                for (int sl = 0; sl < 8; ++sl)
-                    if (nd.meta[sl] & 0x80u) next.push_back((int)nd.child_base + rank++);
+                next.clear();
+                for (int ni : cur)
+                {
+                    level_nodes.push_back(ni);
+                    const ar_wide_node& nd = c.bvh.nodes[ni];
+                    int rank = 0;
+                    for (int sl = 0; sl < 8; ++sl)
+                        if (nd.meta[sl] & 0x80u) next.push_back((int)nd.child_base + rank++);
+                }
+                c.refit_level_off.push_back((int)level_nodes.size());
+                cur.swap(next);
             }
-            c.refit_level_off.push_back((int)level_nodes.size());
-            cur.swap(next);
+            AR_CUDA(ctx, cudaMemcpy(c.d_refit_nodes, level_nodes.data(), level_nodes.size() * sizeof(int), cudaMemcpyHostToDevice));
         }
         std::vector<float> pbox((size_t)std::max(nobj, 1) * 6, 0.0f);
         for (int i = 0; i < nobj; ++i)
             if (c.object_type[i] != AR_OBJECT_TRIANGLE && c.object_type[i] != AR_OBJECT_SDF)
                 object_bounds(c.objects[i], &pbox[6 * (size_t)i], &pbox[6 * (size_t)i + 3]);
-        AR_CUDA(ctx, alloc_dev(c.d_refit_nodes, level_nodes.size()));
-        AR_CUDA(ctx, cudaMemcpy(c.d_refit_nodes, level_nodes.data(), level_nodes.size() * sizeof(int), cudaMemcpyHostToDevice));
         AR_CUDA(ctx, alloc_dev(c.d_mesh_idx, c.mesh_idx.size()));
         AR_CUDA(ctx, cudaMemcpy(c.d_mesh_idx, c.mesh_idx.data(), c.mesh_idx.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
         AR_CUDA(ctx, alloc_dev(c.d_prim_box, pbox.size()));
         AR_CUDA(ctx, cudaMemcpy(c.d_prim_box, pbox.data(), pbox.size() * sizeof(float), cudaMemcpyHostToDevice));
-        AR_CUDA(ctx, alloc_dev(c.d_node_box, 6 * c.bvh.nodes.size()));
+        AR_CUDA(ctx, alloc_dev(c.d_node_box, 6 * (size_t)c.node_count));
     }
     AR_CUDA(ctx, alloc_dev(c.d_objects, objs.size()));
     AR_CUDA(ctx, cudaMemcpy(c.d_objects, objs.data(), objs.size() * sizeof(Object), cudaMemcpyHostToDevice));
@@ -1157,18 +1171,10 @@ ar_status ar_scene_build(ar_ctx* ctx)
         AR_CUDA(ctx, cudaMemcpy(c.d_sdf_nodes, c.sdf_bvh.nodes.data(), c.sdf_bvh.nodes.size() * sizeof(ar_wide_node),
                                 cudaMemcpyHostToDevice));
         AR_CUDA(ctx, alloc_dev(c.d_sdf_bvh_slots, c.sdf_bvh.slots.size() * sizeof(ar_prim_slot)));
-        AR_CUDA(ctx, cudaMemcpy(c.d_sdf_bvh_slots, c.sdf_bvh.slots.data(), c.sdf_bvh.slots.size() * sizeof(ar_prim_slot),
-                                cudaMemcpyHostToDevice));
+        AR_CUDA(ctx, cudaMemcpyAsync(c.d_sdf_bvh_slots, c.sdf_bvh.slots.data(), c.sdf_bvh.slots.size() * sizeof(ar_prim_slot),
+                                     cudaMemcpyHostToDevice, c.stream));
+        AR_CUDA(ctx, launch_slot_tables(c.d_sdf_bvh_slots, (int)c.sdf_bvh.slots.size(), nullptr, nullptr, c.d_prim_slot, c.stream));
     }
-    AR_CUDA(ctx, alloc_dev(c.d_prim_material, (size_t)nprim));
-    AR_CUDA(ctx, cudaMemcpy(c.d_prim_material, prim_material.data(), nprim * sizeof(int), cudaMemcpyHostToDevice));
-    AR_CUDA(ctx, alloc_dev(c.d_prim_light, (size_t)nprim));
-    AR_CUDA(ctx, cudaMemcpy(c.d_prim_light, prim_light.data(), nprim * sizeof(int), cudaMemcpyHostToDevice));
-    AR_CUDA(ctx, alloc_dev(c.d_prim_slot, (size_t)nprim));
-    AR_CUDA(ctx, cudaMemcpy(c.d_prim_slot, prim_slot.data(), nprim * sizeof(int), cudaMemcpyHostToDevice));
-    AR_CUDA(ctx, alloc_dev(c.d_lights, c.lights.size()));
-    if (!c.lights.empty())
-        AR_CUDA(ctx, cudaMemcpy(c.d_lights, c.lights.data(), c.lights.size() * sizeof(Light), cudaMemcpyHostToDevice));
 
     // spectral RGB LUT (2 GiB, built once per context on the GPU)
     if (!c.d_lut_rgb)
@@ -1230,8 +1236,8 @@ ar_status ar_scene_build(ar_ctx* ctx)
     {
         AR_CUDA(ctx, cudaMemcpy(c.d_materials, mats.data(), mats.size() * sizeof(Material), cudaMemcpyHostToDevice));
         AR_CUDA(ctx, launch_prepare_materials(c.d_materials, (int)mats.size(), c.d_lut_rgb, c.stream));
-        AR_CUDA(ctx, cudaStreamSynchronize(c.stream));
     }
+    AR_CUDA(ctx, cudaStreamSynchronize(c.stream));
     c.built = true;
     return AR_OK;
 }
@@ -1277,11 +1283,11 @@ ar_status ar_scene_stats(ar_ctx* ctx, int64_t* n_nodes, int64_t* n_slots, int32_
 {
     if (!ctx) return AR_ERR_INVALID;
     const Ctx& c = ctx->c;
-    if (n_nodes) *n_nodes = (int64_t)c.bvh.nodes.size();
-    if (n_slots) *n_slots = (int64_t)c.bvh.slots.size();
+    if (n_nodes) *n_nodes = c.node_count;
+    if (n_slots) *n_slots = c.slot_count;
     if (depth) *depth = c.bvh.depth;
     if (device_bytes)
-        *device_bytes = (int64_t)(c.bvh.nodes.size() * sizeof(ar_wide_node) + c.bvh.slots.size() * sizeof(ar_prim_slot));
+        *device_bytes = (int64_t)(c.node_count * sizeof(ar_wide_node) + c.slot_count * sizeof(ar_prim_slot));
     return AR_OK;
 }
 
