@@ -254,7 +254,7 @@ struct StageEvent
 
 // Per-path state of the wavefront integrator (structure of arrays).
 // ints in a render wave's counter array (layout: AR_CNT_* in render.cu)
-#define AR_CNT_COUNT 12
+#define AR_CNT_COUNT 16
 
 struct PathState
 {
@@ -335,6 +335,8 @@ struct Ctx
 {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t shadow_stream = nullptr;  // shadow rays beside the next depth's closest hits, between these events
+    cudaEvent_t shade_done = nullptr, shadow_done = nullptr;
     cudaEvent_t order_event = nullptr;  // orders a caller's stream after the context's (ar_render_noalloc)
     // per depth of a wave: the next queue's length, copied to pinned host memory,
     // and the event after the copy (a ring of AR_BOUNCE_LOOKAHEAD + 1)

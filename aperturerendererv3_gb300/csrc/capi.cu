@@ -691,6 +691,9 @@ ar_status ar_create(ar_ctx** out, int device)
     c.device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c.shadow_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c.shade_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c.shadow_done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c.order_event, cudaEventDisableTiming);
     for (int k = 0; k <= AR_BOUNCE_LOOKAHEAD && e == cudaSuccess; ++k)
         e = cudaEventCreateWithFlags(&c.bounce_ev[k], cudaEventDisableTiming);
@@ -748,6 +751,9 @@ ar_status ar_destroy(ar_ctx* ctx)
     free_dev(c.d_frame_dn);
     free_dev(c.d_jumps);
     if (c.order_event) cudaEventDestroy(c.order_event);
+    if (c.shade_done) cudaEventDestroy(c.shade_done);
+    if (c.shadow_done) cudaEventDestroy(c.shadow_done);
+    if (c.shadow_stream) cudaStreamDestroy(c.shadow_stream);
     for (cudaEvent_t& ev : c.bounce_ev)
         if (ev) cudaEventDestroy(ev);
     if (c.h_bounce_cnt) cudaFreeHost(c.h_bounce_cnt);
