@@ -427,21 +427,25 @@ __device__ __forceinline__ void extend_finish(const DevScene& sc, const PathStat
 // the few primitives its cell can need (sdf_cell_mask; 32 primitives before),
 // two lanes share a ray and its primitives, and a warp fetches new rays as soon
 // as a quarter of its lanes have none, so that grazing rays do not hold the rest.
+// The last few rays of a warp, marches of hundreds of steps on an emptying chip,
+// get eight lanes each: one round of distances per step instead of two or three.
 // Terrain with 32 primitives in a medium, 4 samples, depth 24 (all passes and
-// shading): 1280x720 61.0 -> 18.8 ms, 640x360 28.8 -> 9.4, 160x90 14.1 -> 2.9 (the
-// smaller ones with k_finish).  At 640x360 groups of 1 / 2 / 4 / 8 lanes took
+// shading): 1280x720 61.0 -> 15.7 ms, 640x360 28.8 -> 7.2, 320x180 4.9, 160x90 14.1
+// -> 2.9 (with k_finish); without the wide tails 640x360 7.9 (groups of 4 there 7.4, of
+// 16 7.3).  At 640x360 groups of 1 / 2 / 4 / 8 lanes took
 // 13.4 / 11.8 / 11.3 / 13.2 ms, at 1280x720 22.1 / 22.2 / 24.9 / 34.3; 4 blocks per
 // SM 10.9, 3 blocks 11.3.
 #define AR_SDF_GROUP 2        // lanes per ray
 #define AR_SDF_MIN_BLOCKS 4   // blocks per SM the marches are compiled for
-#define AR_SDF_IDLE 4         // idle groups that trigger a refill
-#define AR_SDF_EVALS 4        // evaluations between refill checks
+#define AR_SDF_IDLE 4         // idle groups that trigger a refill (2 and 8 measure alike)
+#define AR_SDF_EVALS 4        // evaluations between refill checks (2 and 8 alike)
+#define AR_SDF_TAIL_GROUP 8   // lanes per ray once a warp's last rays are few (sdf_tail_source)
 
-// sdf_fold by a group of AR_SDF_GROUP lanes with the same p and mask: each
-// lane computes one primitive's distance, every lane folds them in order.
+// sdf_fold by a group of G lanes with the same p and mask: each lane computes one
+// primitive's distance, every lane folds them in order.
+template <int G>
 __device__ __forceinline__ float sdf_fold_group(const SdfUnion& s, unsigned long long mask, V3 p)
 {
-    constexpr int G = AR_SDF_GROUP;
     const int sub = lane_id() & (G - 1), lead = lane_id() & ~(G - 1);
     const unsigned gm = ((1u << G) - 1u) << lead;  // the group's lanes take the same branches
     float d = 0.0f;
@@ -521,10 +525,10 @@ struct SdfMarch
         const V3 e = v3(k < 2 ? h : 0.0f, k == 2 || k == 3 ? h : 0.0f, k >= 4 ? h : 0.0f);
         return (k & 1) ? o - e : o + e;
     }
-    // the field there, by this lane or by the group of lanes that holds this ray
+    // the field there, by this lane or by the group of G lanes that holds this ray
     // (all of them call with the same state); the mask stays while the ray is in
     // one cell
-    template <bool GROUP>
+    template <int G>
     __device__ float field(const SdfUnion& s)
     {
         const V3 p = point();
@@ -534,7 +538,7 @@ struct SdfMarch
             cell = c;
             mask = c >= 0 ? s.cells[c] : sdf_all(s);
         }
-        return GROUP ? sdf_fold_group(s, mask, p) : sdf_fold(s, mask, p);
+        return G > 1 ? sdf_fold_group<G>(s, mask, p) : sdf_fold(s, mask, p);
     }
     // takes the field's value at point(): 0 goes on, 1 no crossing, 2 crossing
     // at t, 3 the normal is complete in g
@@ -563,7 +567,36 @@ struct SdfMarch
         ++n;
         return k == 5 ? 3 : 0;
     }
+    // this march as lane src holds it (a whole warp calls)
+    __device__ void copy_from(int src)
+    {
+        const unsigned all = 0xffffffffu;
+        o = v3(__shfl_sync(all, o.x, src), __shfl_sync(all, o.y, src), __shfl_sync(all, o.z, src));
+        d = v3(__shfl_sync(all, d.x, src), __shfl_sync(all, d.y, src), __shfl_sync(all, d.z, src));
+        g = v3(__shfl_sync(all, g.x, src), __shfl_sync(all, g.y, src), __shfl_sync(all, g.z, src));
+        t = __shfl_sync(all, t, src);
+        t1 = __shfl_sync(all, t1, src);
+        eps = __shfl_sync(all, eps, src);
+        n = __shfl_sync(all, n, src);
+        inside = __shfl_sync(all, (int)inside, src) != 0;
+        cell = -2;
+    }
 };
+
+// The end of a marching kernel: with no ray left to fetch and at most
+// 32 / AR_SDF_TAIL_GROUP in the warp, those rays are spread over its idle lanes.
+// Returns the lane that holds the ray of this lane's wide group (-1: none), or -2
+// while there are more rays or some to fetch.
+__device__ __forceinline__ int sdf_tail_source(bool active, bool exhausted)
+{
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    unsigned leaders = 1u;
+    for (int k = AR_SDF_GROUP; k < 32; k += AR_SDF_GROUP) leaders |= 1u << k;
+    unsigned left = act & leaders;
+    if (!exhausted || __popc(left) > 32 / AR_SDF_TAIL_GROUP) return -2;
+    for (int j = lane_id() / AR_SDF_TAIL_GROUP; j > 0; --j) left &= left - 1u;
+    return left ? __ffs((int)left) - 1 : -1;
+}
 
 // The SDF objects' part of a closest hit (slot, t: the main BVH's): their own
 // BVH, or, for a ray inside one of them (AR_SLOT_SOLO), that object alone.  A hit
@@ -644,6 +677,35 @@ __global__ void __launch_bounds__(AR_BLOCK) k_sdf_objects(DevScene sc, PathState
     }
 }
 
+// Some evaluations of a closest hit's march by its group of G lanes; false when it is done.
+template <int G>
+__device__ __forceinline__ bool sdf_extend_advance(const SdfUnion& un, const PathState& ps, SdfMarch& m, int p, int q, int slot,
+                                                   float& t, float tmin)
+{
+    for (int it = 0; it < AR_SDF_EVALS; ++it)
+    {
+        const int r = m.take(m.field<G>(un));
+        if (r == 0) continue;
+        if (r == 2 && m.t >= tmin && (slot == -1 || m.t < t))
+        {
+            t = m.t;
+            m.begin_normal();
+            continue;
+        }
+        if (r == 3)
+        {
+            // every lane of the group stores the same values
+            const V3 nn = normalize(m.g);
+            ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+            ps.hit_t[p] = t;
+            ps.hit_slot[p] = AR_SLOT_SDF;
+            ps.q_slot[q] = AR_SLOT_SDF;
+        }
+        return false;
+    }
+    return true;
+}
+
 // The smooth union's pass of the closest hits: marched up to the hit so far (it
 // has the largest primitive id, so a hit at equal t wins), and the normal of a
 // hit (central differences of the field), which k_shade reads from hit_nrm.
@@ -677,31 +739,21 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
             if (exhausted) break;
             continue;
         }
-        if (active)
+        const int src = sdf_tail_source(active, exhausted);
+        if (src != -2)
         {
-            for (int it = 0; it < AR_SDF_EVALS; ++it)
-            {
-                const int r = m.take(m.field<true>(un));
-                if (r == 0) continue;
-                if (r == 2 && m.t >= tmin && (slot == -1 || m.t < t))
-                {
-                    t = m.t;
-                    m.begin_normal();
-                    continue;
-                }
-                if (r == 3)
-                {
-                    // every lane of the group stores the same values
-                    const V3 nn = normalize(m.g);
-                    ps.hit_nrm[p] = make_float4(nn.x, nn.y, nn.z, 0.0f);
-                    ps.hit_t[p] = t;
-                    ps.hit_slot[p] = AR_SLOT_SDF;
-                    ps.q_slot[q] = AR_SLOT_SDF;
-                }
-                active = false;
-                break;
-            }
+            const int from = max(src, 0);
+            m.copy_from(from);
+            p = __shfl_sync(0xffffffffu, p, from);
+            q = __shfl_sync(0xffffffffu, q, from);
+            slot = __shfl_sync(0xffffffffu, slot, from);
+            t = __shfl_sync(0xffffffffu, t, from);
+            tmin = __shfl_sync(0xffffffffu, tmin, from);
+            if (src >= 0)
+                while (sdf_extend_advance<AR_SDF_TAIL_GROUP>(un, ps, m, p, q, slot, t, tmin)) {}
+            break;
         }
+        if (active) active = sdf_extend_advance<AR_SDF_GROUP>(un, ps, m, p, q, slot, t, tmin);
     }
 }
 
@@ -1623,6 +1675,21 @@ __global__ void __launch_bounds__(AR_BLOCK) k_sdf_objects_shadow(DevScene sc, Pa
     }
 }
 
+// Some evaluations of a shadow ray's march by its group of G lanes; false when it is done.
+template <int G>
+__device__ __forceinline__ bool sdf_shadow_advance(const SdfUnion& un, const PathState& ps, const ShadowQueue& sq, SdfMarch& m,
+                                                   int i, float tmax, bool lead)
+{
+    for (int it = 0; it < AR_SDF_EVALS; ++it)
+    {
+        const int r = m.take(m.field<G>(un));
+        if (r == 0) continue;
+        if (lead) shadow_apply(ps, sq, i, sq.path[i], r == 2 && m.t >= 0.0f && m.t < tmax);
+        return false;
+    }
+    return true;
+}
+
 __global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
     k_sdf_shadow(SdfUnion un, PathState ps, ShadowQueue sq, SdfPending pend, int* fetch)
 {
@@ -1651,17 +1718,19 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
             if (exhausted) break;
             continue;
         }
-        if (active)
+        const int src = sdf_tail_source(active, exhausted);
+        if (src != -2)
         {
-            for (int it = 0; it < AR_SDF_EVALS; ++it)
-            {
-                const int r = m.take(m.field<true>(un));
-                if (r == 0) continue;
-                if (lead) shadow_apply(ps, sq, i, sq.path[i], r == 2 && m.t >= 0.0f && m.t < tmax);
-                active = false;
-                break;
-            }
+            const int from = max(src, 0);
+            m.copy_from(from);
+            i = __shfl_sync(0xffffffffu, i, from);
+            tmax = __shfl_sync(0xffffffffu, tmax, from);
+            const bool tail_lead = (lane_id() & (AR_SDF_TAIL_GROUP - 1)) == 0;
+            if (src >= 0)
+                while (sdf_shadow_advance<AR_SDF_TAIL_GROUP>(un, ps, sq, m, i, tmax, tail_lead)) {}
+            break;
         }
+        if (active) active = sdf_shadow_advance<AR_SDF_GROUP>(un, ps, sq, m, i, tmax, lead);
     }
 }
 
@@ -1713,18 +1782,17 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_TRAV_MIN_BLOCKS) k_shadow(DevScen
 // resident sets: the launches per depth win above it, where a warp's early-ended
 // lanes stay empty in k_finish but are refilled by the queues.  One frame of the
 // Cornell box, depth 8, launches per depth against k_finish: 256x256 632 -> 332
-// us, 320x320 697 -> 488, 400x400 739 -> 718, 512x512 884 -> 1002.  Glass at depth 1000
+// us, 320x320 697 -> 488, 400x400 739 -> 718, 512x512 884 -> 1002; with shadow rays
+// beside the next depth 320x320 539 -> 478, 384x384 592 -> 590.  Glass at depth 1000
 // with the switch at 1024 per SM: 413x307x8 3.56 -> 1.07 ms, 256x256 1.91 -> 0.36 ms.
 // Blocks of 256 (32 / 64 / 128: 388 / 361 / 348 us for the 256x256 frame, 328 here).
 #define AR_FINISH_BLOCK 256
 #define AR_FINISH_MIN_BLOCKS 2
+// With SDF geometry the line is the same: 320x180x4 (terrain, SDF, medium) 6.9 ms in
+// k_finish and 4.9 by depth, 160x90x4 2.9 and 4.1; 640x360x4 takes 7.2 ms with the
+// switch anywhere from 64 to 1024 paths per SM.  There the warps run apart: a
+// barrier would make each block wait for its longest march.
 #define AR_FINISH_PATHS_PER_SM 1024
-// With SDF geometry every depth waits for its longest marches, twice, so the line
-// lies higher: 640x360x4 (terrain, SDF, medium) 10.1 / 10.0 / 9.4 ms with the switch
-// at 1024 / 2048 / 4096 paths per SM (all of it in k_finish: 21.9), 160x90x4 8.3 ms
-// by depth and 2.9 in k_finish.  There the warps run apart: a barrier would make
-// each block wait for its longest march.
-#define AR_FINISH_SDF_PATHS_PER_SM 4096
 
 // The closest hit of path p's ray: the slot, -1 for none; the distance into
 // hit_t, an SDF hit's normal into hit_nrm.
@@ -1766,7 +1834,7 @@ __device__ __forceinline__ int trace_path(const DevScene& sc, const PathState& p
         if (m.begin(sc.trav.sdf, o, d, sdf_eps(tmin), slot != -1 ? t : 3.0e38f))
         {
             int r;
-            while ((r = m.take(m.field<false>(sc.trav.sdf))) == 0 || (r == 2 && m.t >= tmin && (slot == -1 || m.t < t)))
+            while ((r = m.take(m.field<1>(sc.trav.sdf))) == 0 || (r == 2 && m.t >= tmin && (slot == -1 || m.t < t)))
                 if (r == 2)
                 {
                     t = m.t;
@@ -1794,7 +1862,7 @@ __device__ __forceinline__ bool shadow_path(const DevScene& sc, const ShadowRay&
     SdfMarch m;
     if (!m.begin(sc.trav.sdf, sh.o, sh.d, sdf_eps(0.0f), sh.tmax)) return false;
     int r;
-    while ((r = m.take(m.field<false>(sc.trav.sdf))) == 0) {}
+    while ((r = m.take(m.field<1>(sc.trav.sdf))) == 0) {}
     return r == 2 && m.t >= 0.0f && m.t < sh.tmax;
 }
 
@@ -2167,10 +2235,9 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
     // bound sizes the grids of the queue-sized kernels, so deep bounces with
     // few paths left (or none, at depth limits like 1000) cost launches of a
     // few blocks instead of a wave-sized grid.
-    // k_finish covers scenes without SDF passes and without a guide; profiled
-    // renders keep the stages apart
+    // k_finish covers renders without a guide; profiled ones keep the stages apart
     const bool finish_ok = !rl.guide && c.profile == 0;
-    const long long finish_paths = (long long)sms * (has_sdf ? AR_FINISH_SDF_PATHS_PER_SM : AR_FINISH_PATHS_PER_SM);
+    const long long finish_paths = (long long)sms * AR_FINISH_PATHS_PER_SM;
     constexpr int K = AR_BOUNCE_LOOKAHEAD;
     long long bound = n;  // upper bound of the current depth's queue length
     for (int b = 0; b < rl.max_depth; ++b)
