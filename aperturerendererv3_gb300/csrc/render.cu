@@ -2364,7 +2364,7 @@ cudaError_t launch_render_wave(Ctx& c, const RenderLaunch& rl, long long first_p
 }
 
 // Wave launch over caller-provided buffers (used by the allocation-free entry
-// point); same kernel sequence as launch_render_wave.
+// point): every depth by its launches, all on the caller's stream.
 cudaError_t launch_render_wave_buffers(const DevScene& sc, const WaveBuffers& wb, int device, const RenderLaunch& rl,
                                        int camera_inside, long long first_path, int n, unsigned int* err)
 {

@@ -311,15 +311,16 @@ ar_status ar_trace_any(ar_ctx* ctx, const float* rays, int n, int32_t* hit, void
 #define AR_NOALLOC_MAX_PATHS 40704
 ar_status ar_render_noalloc(ar_ctx* ctx, const ar_render_params* params, double* out_xyz_device, void* stream);
 
-/* Replay adjoint (no counterpart in the reference).  Gradient of a scalar loss
+/* Path adjoint (no counterpart in the reference).  Gradient of a scalar loss
  * with respect to every albedo texel, given dl_dxyz = d(loss)/d(image), where
  * image is what ar_render returns for the same params (per-pixel mean XYZ):
  * device float32, 3 per pixel.  grad_texels: device float64, one per texel
- * float (ar_scene_texel_count), overwritten.  The paths of the render are
- * replayed from their random streams (nothing is stored per vertex): each wave
- * is traced once for its radiance and once more to scatter
+ * float (ar_scene_texel_count), overwritten.  The paths of the render are traced
+ * again from their random streams, a wave at a time, with 8 bytes recorded per
+ * vertex (at most 1 GiB, kept with the context; a wave that needs more, or finds no
+ * memory for them, is traced twice instead and records nothing), and
  * d(loss)/d(radiance) x (radiance still to come) x d(albedo)/d(texel) / albedo
- * at every textured diffuse vertex.  Russian-roulette and NEE decisions are
+ * is added for every textured diffuse vertex.  Russian-roulette and NEE decisions are
  * held fixed (their probabilities are not differentiated).  Gradients gather
  * in float32 per wave and fold into grad_texels in float64.  Guided rendering
  * is rejected. */
