@@ -28,6 +28,7 @@
 
 #include "../../include/aperture/ar.h"
 #include "ar_bvh_build.h"
+#include "ar_bvh_lanes.h"
 #include "ar_internal.h"
 
 namespace ar
@@ -354,14 +355,6 @@ __global__ void k_boxes(const arbvh::PrimInput* __restrict__ prims, const unsign
     }
 }
 
-__device__ __forceinline__ double box_area(const Box6& b)
-{
-    const double dx = fmax(0.0, (double)b.hi[0] - b.lo[0]);
-    const double dy = fmax(0.0, (double)b.hi[1] - b.lo[1]);
-    const double dz = fmax(0.0, (double)b.hi[2] - b.lo[2]);
-    return 2.0 * (dx * dy + dy * dz + dz * dx);
-}
-
 // number of sorted primitives under binary node b
 __device__ __forceinline__ int node_count(int b, int n, const int2* range)
 {
@@ -416,7 +409,8 @@ __device__ __forceinline__ uint8_t quant_high(float hi, float node_lo, float inv
 // One wide node per 8 lanes, one lane per child (lane k of a group: child k, then
 // slot k).  A node by a single thread is a serial chain of some 1,500 double
 // precision operations and its local arrays; by a group it is a few rounds of
-// shuffles (200,000 triangles, 7 levels: 1068 -> 256 us).  queue: (wide index,
+// shuffles (200,000 triangles, 7 levels: 1068 -> 256 us).  All lanes of a group have
+// to end each round with the same winner (ar_bvh_lanes.h).  queue: (wide index,
 // binary index); internal children are appended to the next level's queue.
 __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __restrict__ queue, int nq, int2* next,
                                                 int* next_count, unsigned int* err)
@@ -446,7 +440,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __
     if (ch >= 0)
     {
         cb = a.box[ch];
-        if (cnt > kMaxLeaf) area = box_area(cb);
+        if (cnt > kMaxLeaf) area = open_area(cb.lo, cb.hi);
     }
     while (nch < 8)
     {
@@ -456,7 +450,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __
         {
             const double o = __shfl_xor_sync(gm, best, k);
             const int p = __shfl_xor_sync(gm, pick, k);
-            if (o > best || (o == best && p < pick))
+            if (opens_before(o, p, best, pick))
             {
                 best = o;
                 pick = p;
@@ -470,7 +464,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __
             ch = sub == pick ? cc.x : cc.y;
             cnt = node_count(ch, n, a.range);
             cb = a.box[ch];
-            area = cnt > kMaxLeaf ? box_area(cb) : -1.0;
+            area = cnt > kMaxLeaf ? open_area(cb.lo, cb.hi) : -1.0;
         }
         ++nch;
     }
@@ -501,8 +495,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __
             for (int s = 0; s < 8; ++s)
             {
                 if ((taken >> s) & 1u) continue;
-                double c = 0.0;
-                for (int k = 0; k < 3; ++k) c += ((s >> k) & 1) ? off[k] : -off[k];
+                const double c = slot_cost(off, s);
                 if (bs == 8 || c > bc)
                 {
                     bc = c;
@@ -515,7 +508,7 @@ __global__ void __launch_bounds__(128) k_collapse(CollapseArgs a, const int2* __
             const double o = __shfl_xor_sync(gm, bc, k);
             const int w = __shfl_xor_sync(gm, who, k);
             const int s = __shfl_xor_sync(gm, bs, k);
-            if (w < 8 && (who >= 8 || o > bc || (o == bc && w < who)))
+            if (placed_before(o, w, bc, who))
             {
                 bc = o;
                 who = w;
