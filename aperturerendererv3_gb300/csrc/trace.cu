@@ -6,6 +6,7 @@
 #include <algorithm>
 
 #include "ar_internal.h"
+#include "ar_ray_share.h"
 
 namespace ar
 {
@@ -31,11 +32,9 @@ __global__ void __launch_bounds__(TR_BLOCK, TR_BLOCKS) k_trace_rays(TravScene sc
                                                                    float* __restrict__ tout, unsigned int* err)
 {
     const int lane = threadIdx.x & 31;
-    const int warps = gridDim.x * (TR_BLOCK / 32), w = blockIdx.x * (TR_BLOCK / 32) + (threadIdx.x >> 5);
-    const int chunk = 1 << chunk_log2;
-    // the warp's rays in order: local index j is ray ((j / chunk) warps + w) chunk + j % chunk
-    const int chunks = (n + chunk - 1) >> chunk_log2;
-    const int limit = w < chunks ? ((chunks - w - 1) / warps + 1) << chunk_log2 : 0;
+    const int w = blockIdx.x * (TR_BLOCK / 32) + (threadIdx.x >> 5);
+    const RayShare share{n, chunk_log2, (int)gridDim.x * (TR_BLOCK / 32)};
+    const int limit = share.limit(w);
     int next = 0;
     TravState<AnyHit> st;
     uint2 stk[AR_TRAV_STACK];
@@ -49,7 +48,7 @@ __global__ void __launch_bounds__(TR_BLOCK, TR_BLOCKS) k_trace_rays(TravScene sc
             if (!active)
             {
                 const int j = next + __popc(idle & ((1u << lane) - 1u));
-                const long long r = ((long long)(j >> chunk_log2) * warps + w) * chunk + (j & (chunk - 1));
+                const long long r = share.ray(w, j);
                 if (j < limit && r < n)
                 {
                     i = (int)r;
@@ -145,7 +144,7 @@ cudaError_t launch_trace(const DevScene& sc, const float* rays, int n, int any, 
         const long long resident = (long long)sms * (1024 / 32);  // warps
         int chunk_log2 = 0;
         while (chunk_log2 < 5 && ((long long)n >> chunk_log2) > resident / 2) ++chunk_log2;
-        const long long chunks = ((long long)n + (1 << chunk_log2) - 1) >> chunk_log2;
+        const long long chunks = RayShare{n, chunk_log2, 1}.chunks();
         const int grid = (int)((std::min(chunks, resident) + TR_BLOCK / 32 - 1) / (TR_BLOCK / 32));
         if (any) k_trace_rays<true><<<grid, TR_BLOCK, 0, s>>>(sc.trav, r4, n, chunk_log2, prim_id, nullptr, err);
         else k_trace_rays<false><<<grid, TR_BLOCK, 0, s>>>(sc.trav, r4, n, chunk_log2, prim_id, t, err);
