@@ -415,7 +415,7 @@ struct Ctx
     long long grad32_n = 0;
     float* d_adj = nullptr;              // 2 floats per wave path
     int adj_capacity = 0;
-    int2* d_adj_rec = nullptr;           // recording pass: one record per depth and path of a wave
+    int2* d_adj_rec = nullptr;           // recording pass: one record per depth and path; freed with the waves
     size_t adj_rec_n = 0;
     double* d_grad_medium = nullptr;     // d loss / d (medium albedo, medium emission)
     // smooth-union SDF object and the participating medium

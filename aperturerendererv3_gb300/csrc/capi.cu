@@ -170,6 +170,8 @@ void free_waves(Ctx& c)
     free_dev(c.d_queue[0]);
     free_dev(c.d_queue[1]);
     free_dev(c.d_pq);
+    free_dev(c.d_adj_rec);  // sized by a wave as well
+    c.adj_rec_n = 0;
     c.wave_capacity = 0;
     p.capacity = 0;
 }
@@ -745,7 +747,6 @@ ar_status ar_destroy(ar_ctx* ctx)
     free_dev(c.d_stats);
     free_dev(c.d_grad32);
     free_dev(c.d_adj);
-    free_dev(c.d_adj_rec);
     free_dev(c.d_grad_medium);
     free_dev(c.d_frame_xyz);
     free_dev(c.d_frame_dn);
@@ -1460,6 +1461,18 @@ ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_
     if ((long long)cap > total) cap = (int)total;
     st = ensure_waves(ctx, cap);
     if (st != AR_OK) return st;
+    if (grad_texels)
+    {
+        if (c.grad32_n < c.texel_floats)
+        {
+            free_dev(c.d_grad32);
+            AR_CUDA(ctx, alloc_dev(c.d_grad32, (size_t)c.texel_floats));
+            AR_CUDA(ctx, cudaMemset(c.d_grad32, 0, (size_t)c.texel_floats * sizeof(float)));
+            c.grad32_n = c.texel_floats;
+        }
+        AR_CUDA(ctx, cudaMemsetAsync(grad_texels, 0, (size_t)c.texel_floats * sizeof(double), c.stream));
+    }
+    // the records last, so that they leave room for what the replay needs too
     const long long records = (long long)cap * rl.max_depth;
     bool record = grad_texels && records <= AR_ADJ_RECORDS_MAX;
     if (record && c.adj_rec_n < (size_t)records)
@@ -1483,17 +1496,6 @@ ar_status run_adjoint(ar_ctx* ctx, const ar_render_params* prm, const float* dl_
     }
     c.ps.adj_total = c.d_adj;
     c.ps.adj_delta = c.d_adj ? c.d_adj + c.ps.capacity : nullptr;
-    if (grad_texels)
-    {
-        if (c.grad32_n < c.texel_floats)
-        {
-            free_dev(c.d_grad32);
-            AR_CUDA(ctx, alloc_dev(c.d_grad32, (size_t)c.texel_floats));
-            AR_CUDA(ctx, cudaMemset(c.d_grad32, 0, (size_t)c.texel_floats * sizeof(float)));
-            c.grad32_n = c.texel_floats;
-        }
-        AR_CUDA(ctx, cudaMemsetAsync(grad_texels, 0, (size_t)c.texel_floats * sizeof(double), c.stream));
-    }
     if (grad_medium) AR_CUDA(ctx, cudaMemsetAsync(grad_medium, 0, 2 * sizeof(double), c.stream));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);

@@ -317,7 +317,7 @@ ar_status ar_render_noalloc(ar_ctx* ctx, const ar_render_params* params, double*
  * device float32, 3 per pixel.  grad_texels: device float64, one per texel
  * float (ar_scene_texel_count), overwritten.  The paths of the render are traced
  * again from their random streams, a wave at a time, with 8 bytes recorded per
- * vertex (at most 1 GiB, kept with the context; a wave that needs more, or finds no
+ * vertex (at most 1 GiB, kept with the wave buffers; a wave that needs more, or finds no
  * memory for them, is traced twice instead and records nothing), and
  * d(loss)/d(radiance) x (radiance still to come) x d(albedo)/d(texel) / albedo
  * is added for every textured diffuse vertex.  Russian-roulette and NEE decisions are
