@@ -6,7 +6,8 @@
 //   w0: origin p.xyz (f32) | exponents ex, ey, ez (u8, biased 127) | internal-child mask (u8)
 //   w1: child_base (u32) | prim_base (u32) | meta[0..7] (u8)
 //   w2: qlo_x[8], qlo_y[8]      w3: qlo_z[8], qhi_x[8]      w4: qhi_y[8], qhi_z[8]
-// A child box decodes as p + q * 2^(e-127) per axis (exact conservative bounds).
+// A child box decodes as p + q * 2^(e-127) per axis (exact conservative bounds), with
+// e - 127 >= AR_BVH_MIN_EXP also where a node is thinner or flat.
 // meta[i]: 0 = empty slot (its box is inverted, qlo 255 and qhi 0: no ray meets it);
 //          0x80 | r = internal child stored at child_base + r;
 //          (n << 5) | off = leaf with n (1..3) primitive slots at prim_base + off.
@@ -21,6 +22,11 @@
 #include <stdint.h>
 
 #define AR_BVH_WIDTH 8
+// Smallest quantisation step, 2^-64: the slab test's margin for an axis-parallel ray is
+// 2^-8 of a step times 2^104 (slab_inv), so such a ray reaches t = 2^30 inside a slab
+// however thin.  Scenes smaller than 255 steps, 1.4e-17 units, are traced without
+// culling.
+#define AR_BVH_MIN_EXP (-64)
 #define AR_PRIM_KIND_SHIFT 30
 #define AR_PRIM_KIND_TRI 0u
 #define AR_PRIM_KIND_BOX 1u

@@ -170,16 +170,13 @@ AR_HD bool packet_child_meets(const uint4& w0, const uint4& w1, const uint4& w2,
 #define AR_DEVERR_QUEUE 2u
 
 // Reciprocal of a direction component for the slab test: a zero component takes
-// 2^96, so that an axis-parallel ray still tells the slabs it lies in from those
-// beside it (in nodes up to e = 15; above, that axis keeps every child).
-AR_HD float slab_inv(float x) { return x == 0.0f ? 0x1p96f : 1.0f / x; }
+// 2^104, so that an axis-parallel ray still tells the slabs it lies in from those
+// beside it (in nodes up to e = 8 and 2^24 units away; beyond, that axis keeps every
+// child) and its margin there passes t (AR_BVH_MIN_EXP).
+AR_HD float slab_inv(float x) { return x == 0.0f ? 0x1p104f : 1.0f / x; }
 
-// Margin of a node's planes on one axis, from the offsets B and C of
-// TravState::step and the reciprocal 1 / d.
-AR_HD float slab_margin(float b, float c, float inv)
-{
-    return fmaf(fabsf(c), 0x1.4p-23f, fmaf(fabsf(b), 0x1p-21f, fabsf(inv) * 0x1p-64f));
-}
+// Margin of a node's planes on one axis, from the offsets B and C of TravState::step.
+AR_HD float slab_margin(float b, float c) { return fmaf(fabsf(c), 0x1.4p-23f, fabsf(b) * 0x1p-21f); }
 
 // Two children's values side by side.  On the device one packed fused
 // multiply-add (fma.rn.f32x2) takes one issue slot for both; each half rounds
@@ -337,7 +334,7 @@ struct TravState
             // which is one byte permute (the byte under the exponent of 2^15)
             // where extracting and converting it takes two instructions, so
             // the offset is C = B - 32768 A and each plane one fused
-            // multiply-add.  E = 1.25 2^-23 |C| + 2^-21 |B| + 2^-64 / |d| bounds every
+            // multiply-add.  E = 1.25 2^-23 |C| + 2^-21 |B| bounds every
             // rounding, in units of 2^-24: 4 |B| (the difference, the reciprocal, the
             // product, the plane), 2 |C| (C and C -+ E) and 512 |A| (the reciprocal
             // and the plane of steps up to 255), where 32768 |A| <= |B| + |C|; it is
@@ -346,17 +343,14 @@ struct TravState
             // ray meets.  The margin has to follow C: where 32768 |A| overflows, C is
             // infinite while A and B need not be, and then so is E, which makes
             // C - E and C + E infinite on the permissive side or NaN, which the min /
-            // max ignore.  The last term lets an axis-parallel ray reach t = 2^32 in
-            // slabs however thin (the far plane of one it lies in may be at 0 2^96);
-            // for other rays it is 2^-64 of a length unit.  It costs one multiplication
-            // per axis and node: 2.07 M rays against 1M random triangles 1.78 -> 1.80 ms,
-            // 1080p terrain 34.2 ms with and without.  The near plane of each axis is
-            // the low one when the direction is positive (octant bit clear): no min /
-            // max pairs.
+            // max ignore (the margin from A, finite there, measures the same: 2.07 M rays
+            // against 1M random triangles 1.78 ms).  The near plane of each axis is the
+            // low one when the direction is positive (octant bit clear): no min / max
+            // pairs.
             const float ax = sx * inv.x, ay = sy * inv.y, az = sz * inv.z;
             const float bx = (px - o.x) * inv.x, by = (py - o.y) * inv.y, bz = (pz - o.z) * inv.z;
             const float cx = fmaf(-32768.0f, ax, bx), cy = fmaf(-32768.0f, ay, by), cz = fmaf(-32768.0f, az, bz);
-            const float ex = slab_margin(bx, cx, inv.x), ey = slab_margin(by, cy, inv.y), ez = slab_margin(bz, cz, inv.z);
+            const float ex = slab_margin(bx, cx), ey = slab_margin(by, cy), ez = slab_margin(bz, cz);
             const bool fx = oct & 1u, fy = oct & 2u, fz = oct & 4u;
             const uint32_t nx0 = fx ? w3.z : w2.x, nx1 = fx ? w3.w : w2.y, fx0 = fx ? w2.x : w3.z, fx1 = fx ? w2.y : w3.w;
             const uint32_t ny0 = fy ? w4.x : w2.z, ny1 = fy ? w4.y : w2.w, fy0 = fy ? w2.z : w4.x, fy1 = fy ? w2.w : w4.y;

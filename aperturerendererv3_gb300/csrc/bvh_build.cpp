@@ -281,12 +281,12 @@ struct Collapser
         for (int k = 0; k < 3; ++k)
         {
             const double ext = (double)nb.hi[k] - nb.lo[k];
-            int e = -126;
+            int e = AR_BVH_MIN_EXP;
             if (ext > 0.0)
             {
                 e = (int)std::ceil(std::log2(ext / 255.0));
                 while (std::ldexp(255.0, e) < ext) ++e;
-                e = std::max(-126, std::min(127, e));
+                e = std::max(AR_BVH_MIN_EXP, std::min(127, e));
             }
             node.e[k] = (uint8_t)(e + 127);
             scale[k] = (float)std::ldexp(1.0, e);

@@ -383,16 +383,16 @@ struct CollapseArgs
 };
 
 // Exponent e (biased by 127 in a node) of the smallest power of two with
-// 255 2^e >= hi - lo, at least 2^-126: the difference rounded up is m 2^k with m in
+// 255 2^e >= hi - lo, at least AR_BVH_MIN_EXP: the difference rounded up is m 2^k with m in
 // [1, 2), and 255 is 1.9921875 2^7.
 __device__ __forceinline__ int quant_exponent(float lo, float hi)
 {
     const float ext = __fsub_ru(hi, lo);
-    if (!(ext > 0.0f)) return -126;
+    if (!(ext > 0.0f)) return AR_BVH_MIN_EXP;
     const uint32_t u = __float_as_uint(ext);
     const int k = (int)(u >> 23) - 127;
     const int e = k - 7 + ((u & 0x7fffffu) > 0x7f0000u || k == 128 ? 1 : 0);
-    return e < -126 ? -126 : e;
+    return e < AR_BVH_MIN_EXP ? AR_BVH_MIN_EXP : e;
 }
 
 // A child plane in steps of 2^e above the node's low plane, moved outwards: the

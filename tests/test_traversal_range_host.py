@@ -6,8 +6,8 @@ which overflows for large nodes and for small direction components.  A box that 
 ray meets in [tmin, tlim] may not be rejected there: the traversal's own step()
 runs against random nodes with steps from 2^-126 to 2^120 and rays with ordinary,
 zero, negative zero, subnormal and tiny components, and is compared with a slab
-test in double precision; sheets of 1 to 1e8 units are compared with a test of
-every triangle in double precision."""
+test in double precision; sheets of 1 to 1e12 units, some of them squashed to
+ribbons, are compared with a test of every triangle in double precision."""
 import ctypes as C
 import os
 import shutil
@@ -63,11 +63,11 @@ int main()
         ar_wide_node nd;
         std::memset(&nd, 0, sizeof(nd));
         int e[3];
-        const int base = kind == THIN ? -30 + (int)(U(rng) * 40) : -126 + (int)(U(rng) * 246);
+        const int base = kind == THIN ? -30 + (int)(U(rng) * 30) : -126 + (int)(U(rng) * 246);
         for (int k = 0; k < 3; ++k)
         {
-            // THIN: a node of any extent along the axis that the ray is perpendicular to
-            e[k] = kind == THIN && k == ax ? -126 + (int)(U(rng) * (base + 126))
+            // THIN: a node of any extent that is built along the axis that the ray is perpendicular to
+            e[k] = kind == THIN && k == ax ? AR_BVH_MIN_EXP + (int)(U(rng) * (base - AR_BVH_MIN_EXP))
                                            : std::min(119, std::max(-126, base + (int)(U(rng) * 10) - 5));
             nd.e[k] = (uint8_t)(e[k] + 127);
         }
@@ -176,10 +176,10 @@ def test_no_box_is_rejected_at_any_scale(tmp_path):
         assert missed == 0, f"{kind}: {missed} of {met} boxes that the ray meets were rejected"
 
 
-def sheet(size, n=24):
-    """n x n quads of two triangles each over [-size, size]^2 at y = 0, (2 n^2, 9)."""
+def sheet(size, n=24, thin=1.0):
+    """n x n quads of two triangles each over [-size, size]^2 at y = 0, (2 n^2, 9), x scaled by thin."""
     g = np.linspace(-size, size, n + 1)
-    x, z = np.meshgrid(g, g, indexing="ij")
+    x, z = np.meshgrid(thin * g, g, indexing="ij")
     v = np.stack([x, np.zeros_like(x), z], -1)
     a, b, c, d = v[:-1, :-1], v[1:, :-1], v[1:, 1:], v[:-1, 1:]
     return np.concatenate([np.stack([a, b, c], 2).reshape(-1, 9), np.stack([a, c, d], 2).reshape(-1, 9)]).astype(np.float32)
@@ -217,14 +217,30 @@ def every_triangle(tris, rays):
     return np.where(np.isfinite(best), i, -1).astype(np.int32), best
 
 
-SHEETS = [(1.0, (0.0, -1.0, 0.0)), (1.0, (1e-36, -1.0, 0.3)), (1e3, (1e-36, -1.0, 0.3)), (1e3, (-1e-37, -1.0, -1e-40)),
-          (1e7, (1e-30, -1.0, 1e-30)), (8e6, (0.0, -1.0, 0.0)), (9e6, (0.0, -1.0, 0.0)), (9e6, (1e-3, -1.0, 0.0)),
-          (1e8, (0.0, -1.0, 0.0)), (1e8, (-0.0, -1.0, 0.25)), (1e8, (0.5, -1.0, 0.25)), (1e12, (0.0, -1.0, 1e-20))]
+# size, direction, scale of x
+SHEETS = [
+    (1.0, (0.0, -1.0, 0.0), 1.0),
+    (1.0, (1e-36, -1.0, 0.3), 1.0),
+    (1e3, (1e-36, -1.0, 0.3), 1.0),
+    (1e3, (-1e-37, -1.0, -1e-40), 1.0),
+    (1e7, (1e-30, -1.0, 1e-30), 1.0),
+    (8e6, (0.0, -1.0, 0.0), 1.0),
+    (9e6, (0.0, -1.0, 0.0), 1.0),
+    (9e6, (1e-3, -1.0, 0.0), 1.0),
+    (1e8, (0.0, -1.0, 0.0), 1.0),
+    (1e8, (-0.0, -1.0, 0.25), 1.0),
+    (1e8, (0.5, -1.0, 0.25), 1.0),
+    (1e12, (0.0, -1.0, 1e-20), 1.0),
+    (1.0, (0.0, -1.0, 0.0), 1e-12),
+    (1.0, (0.0, -1.0, 0.0), 1e-25),
+    (1.0, (0.0, -1.0, 0.5), 1e-30),
+    (1e6, (0.0, -1.0, 0.0), 1e-31),
+]
 
 
-@pytest.mark.parametrize("size,direction", SHEETS)
-def test_sheets_answer_as_every_triangle(size, direction):
-    tris = sheet(size)
+@pytest.mark.parametrize("size,direction,thin", SHEETS)
+def test_sheets_answer_as_every_triangle(size, direction, thin):
+    tris = sheet(size, thin=thin)
     rays = sheet_rays(tris, direction, 0.5 * size)
     want, want_t = every_triangle(tris, rays)
     assert (want >= 0).all()
