@@ -1,4 +1,4 @@
-// Replay adjoint of the albedo textures (no counterpart in the reference).
+// Path adjoint of the albedo textures (no counterpart in the reference).
 //
 // ar_adjoint renders every wave once, with shading (k_shade<0, AR_ADJ_RECORD, *>)
 // leaving per vertex the texel whose colour it used and the radiance of the path

@@ -1577,13 +1577,15 @@ __device__ __forceinline__ void add_medium_gradient(double* grad_medium, float g
 // none).  More barriers gain nothing further.
 //
 // Threads per block, two blocks on an SM: shading waits on instruction fetch and
-// on scattered loads, so the leaner instantiations, which spill little at fewer
-// registers, do better with more warps. Measured on the stage's time: opaque
+// on scattered loads, so the leaner instantiations do better with more warps even
+// where they spill: opaque untextured 80 registers with 260 / 208 bytes of spill
+// stores / loads, with the voxel guide 72 with 452 / 664. On the stage's time: opaque
 // untextured (1080p terrain) 10.0 ms at 256 threads, 9.2 at 320, 8.8 at 384, 8.9 at
 // 448; the same with the voxel guide (480 x 270) 3.75 ms at 256, 3.5 at 320, 3.6 at
 // 384, 3.3 at 448. The others keep 256: textured 256 x 256 with its replay 22.8 ms
 // for a whole step, 23.1 at 320, 23.7 at 384, and the full set of materials spills
-// at 128 registers already.
+// at 128 registers already (20 / 20 bytes unguided, 56 / 84 with the voxel guide,
+// 372 / 344 with the network).
 template <int GUIDE, int ADJ, int FEAT>
 constexpr int kShadeBlock = FEAT != AR_FEAT_SURFACE ? 256 : GUIDE ? 448 : 384;
 constexpr int AR_SHADE_RESIDENT = 2;  // blocks on an SM

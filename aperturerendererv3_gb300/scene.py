@@ -651,6 +651,9 @@ class SceneRenderer:
         return n.value, loss.value
 
     def render_profile(self) -> dict:
+        """Stage times and counters of the last render with profile=1, 2 or 3.  A profiled render keeps its stages
+        apart: a plain one takes few paths to their end in one launch and traces shadow rays beside the next
+        depth's closest hits, so its time is not the sum of these."""
         prof = _lib.ArRenderProfile()
         check(self._ctx, self._lib.ar_last_render_profile(self._ctx, C.byref(prof)))
         return prof.as_dict()

@@ -1,4 +1,4 @@
-"""PyTorch binding of the replay adjoint: rendering as a differentiable function
+"""PyTorch binding of the path adjoint: rendering as a differentiable function
 of the albedo texels.
 
     img = render_textures(texels, renderer, (W, H), origin, direction, spp, fov=40, max_depth=8)
@@ -7,8 +7,10 @@ of the albedo texels.
 
 Forward uploads the texels into the renderer's scene and renders the per-pixel
 mean XYZ (float64, on the texels' device).  Backward re-uploads the texels the
-forward saw and calls the C ABI's replay adjoint with d(loss)/d(image); the
-gradient comes back as float64 sums and is cast to the texels' dtype.  Both
+forward saw and calls ar_adjoint with d(loss)/d(image), which traces the same
+paths again, recording their vertices (or, where a wave's paths times the depth
+limit pass 2^27 records, tracing them twice); the gradient comes back as float64
+sums and is cast to the texels' dtype.  Both
 directions go through the same C entry points a C++ caller would use; there is
 no Python or CPU fallback.
 """

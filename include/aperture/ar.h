@@ -108,7 +108,8 @@ typedef struct ar_render_params
     int32_t first_frame;     /* frame index of the first sample */
     int32_t wave_paths;      /* paths in flight per wave, 0 = automatic (ar_render: up to 2^25,
                                 about 8 GB of device state; ar_adjoint: up to 2^21) */
-    int32_t profile;         /* 1 = per-stage device times, 2 = traversal counters, 3 = both */
+    int32_t profile;         /* 1 = per-stage device times, 2 = traversal counters, 3 = both; any of them keeps
+                                the stages apart (ar_render_profile) */
     int32_t guide;           /* AR_GUIDE_NONE, AR_GUIDE_VOXEL (SceneSetting::bUsePathGuiding_) or AR_GUIDE_MLP */
     float guide_unit;        /* voxel size of the guide (0 = 0.05, PATH_GUIDING_RESOLUTION_UNIT) */
     int32_t guide_train_steps; /* AR_GUIDE_MLP: Adam steps after each frame (0 = 8) */
@@ -136,7 +137,10 @@ typedef struct ar_render_params
  * network's 64-cell directional distribution; later bounces keep the probes. */
 #define AR_GUIDE_MLP 2
 
-/* Per-stage profile of the last ar_render with params->profile = 1. */
+/* Per-stage profile of the last ar_render with params->profile = 1.  A profiled
+ * render gives the same image by other launches than a plain one: every depth is
+ * traced and shaded by launches of its own, however few paths are left, and its
+ * shadow rays are traced before the next depth's closest hits, not beside them. */
 typedef struct ar_render_profile
 {
     float raygen_ms, extend_ms, shade_ms, shadow_ms, finalize_ms;
