@@ -25,11 +25,13 @@ struct TravScene
 {
     const uint4* __restrict__ nodes;       // 5 uint4 per node
     const float4* __restrict__ slots;      // 3 float4 per primitive slot
-    const Object* __restrict__ objects;    // analytic object table, indexed by primitive id
+    const Object* __restrict__ objects;    // object table, indexed by primitive id below object_count
+                                           // (mesh triangles and the union follow and are not in it)
     const float4* __restrict__ sdf_params; // SDF objects: field parameters, indexed by primitive id
     const SdfVolume* __restrict__ sdf_vols;  // the SDF volume cache
     int sdf_vol_count;
     int node_count;
+    int object_count;
     SdfUnion sdf;                          // the smooth-union SDF object (count 0: none); not in the BVH
     int sdf_id;                            // its primitive id
 };

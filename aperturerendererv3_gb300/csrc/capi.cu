@@ -32,6 +32,7 @@ DevScene dev_scene(const Ctx& c)
     s.trav.nodes = reinterpret_cast<const uint4*>(c.d_nodes);
     s.trav.slots = reinterpret_cast<const float4*>(c.d_slots);
     s.trav.objects = c.d_objects;
+    s.trav.object_count = (int)c.objects.size();
     s.trav.sdf_params = c.d_sdf_params;
     s.trav.sdf_vols = c.d_vols;
     s.trav.sdf_vol_count = (int)c.vol_dev.size();
@@ -1852,6 +1853,7 @@ ar_status ar_host_trace_closest(const float* tris, int ntri, const float* rays, 
     sc.nodes = reinterpret_cast<const uint4*>(bvh.nodes.data());
     sc.slots = reinterpret_cast<const float4*>(bvh.slots.data());
     sc.objects = nullptr;
+    sc.object_count = 0;
     sc.sdf_params = nullptr;
     sc.sdf_vols = nullptr;
     sc.sdf_vol_count = 0;

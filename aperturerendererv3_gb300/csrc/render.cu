@@ -598,6 +598,25 @@ __device__ __forceinline__ int sdf_tail_source(bool active, bool exhausted)
     return left ? __ffs((int)left) - 1 : -1;
 }
 
+// The object a ray is inside of, as the path's media record has it, may be any
+// primitive: a path that starts in one (the camera inside an object) takes the
+// last surface it left.  Rays inside an SDF object test it in the SDF pass.
+__device__ __forceinline__ bool inside_sdf_object(const Object* objects, int object_count, int id)
+{
+    return id >= 0 && id < object_count && objects[id].type == AR_OBJ_SDF;
+}
+
+// Rays inside any other: the hit on it alone, its slot or -1 and t.  The union has
+// no slot; its own pass marches it.
+__device__ __forceinline__ int enclosing_hit(const DevScene& sc, int id, V3 o, V3 d, float tmin, float* t)
+{
+    const int s = sc.prim_slot[id];
+    int hit_id;
+    const float th = s >= 0 ? prim_hit<false>(sc.trav, s, make_shear(d), o, d, &hit_id, tmin) : -1.0f;
+    *t = th >= tmin ? th : 0.0f;
+    return th >= tmin ? s : -1;
+}
+
 // The SDF objects' part of a closest hit (slot, t: the main BVH's): their own
 // BVH, or, for a ray inside one of them (AR_SLOT_SOLO), that object alone.  A hit
 // on one replaces slot and t and leaves its normal in hit_nrm.  Returns whether
@@ -711,7 +730,7 @@ __device__ __forceinline__ bool sdf_extend_advance(const SdfUnion& un, const Pat
 // hit (central differences of the field), which k_shade reads from hit_nrm.
 // Rays inside an SDF object test only that object (objects: null without any).
 __global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
-    k_sdf_extend(SdfUnion un, const Object* __restrict__ objects, PathState ps, const int* __restrict__ queue,
+    k_sdf_extend(SdfUnion un, const Object* __restrict__ objects, int object_count, PathState ps, const int* __restrict__ queue,
                  const int* __restrict__ counter, int* fetch)
 {
     const int n = *counter;
@@ -730,7 +749,7 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_SDF_MIN_BLOCKS)
             slot = ps.hit_slot[p];
             t = ps.hit_t[p];
             const int mobj = objects && (ps.flags[p] & 1u) ? __float_as_int(ps.media_v[p].w) : -1;
-            const bool solo = mobj >= 0 && objects[mobj].type == AR_OBJ_SDF;
+            const bool solo = inside_sdf_object(objects, object_count, mobj);
             active = !solo && m.begin(un, v3(ro.x, ro.y, ro.z), v3(rd.x, rd.y, rd.z), sdf_eps(tmin),
                                       slot != -1 ? t : 3.0e38f);
         }
@@ -781,7 +800,7 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_TRAV_MIN_BLOCKS) k_extend(DevScen
             {
                 // inside a medium: intersect only the enclosing object (render.cuh:89-92);
                 // an SDF object is left to the SDF pass
-                if (sc.trav.objects[mobj].type == AR_OBJ_SDF)
+                if (inside_sdf_object(sc.trav.objects, sc.trav.object_count, mobj))
                 {
                     ps.hit_t[p] = 0.0f;
                     ps.hit_slot[p] = AR_SLOT_SOLO;
@@ -789,12 +808,11 @@ __global__ void __launch_bounds__(AR_BLOCK, AR_TRAV_MIN_BLOCKS) k_extend(DevScen
                 }
                 else
                 {
-                    const int s = sc.prim_slot[mobj];
-                    int id;
-                    const float th = prim_hit<false>(sc.trav, s, make_shear(d), o, d, &id, tmin);
-                    ps.hit_t[p] = th >= tmin ? th : 0.0f;
-                    ps.hit_slot[p] = th >= tmin ? s : -1;
-                    ps.q_slot[q] = th >= tmin ? s : -1;
+                    float th;
+                    const int s = enclosing_hit(sc, mobj, o, d, tmin, &th);
+                    ps.hit_t[p] = th;
+                    ps.hit_slot[p] = s;
+                    ps.q_slot[q] = s;
                 }
                 if (sc.stats) atomicAdd(&sc.stats[4], 1ull);
             }
@@ -1810,19 +1828,12 @@ __device__ __forceinline__ int trace_path(const DevScene& sc, const PathState& p
     if (mobj >= 0)
     {
         // inside a medium: only the enclosing object (as in k_extend)
-        if (SDF && sc.trav.objects[mobj].type == AR_OBJ_SDF)
+        if (SDF && inside_sdf_object(sc.trav.objects, sc.trav.object_count, mobj))
         {
             slot = AR_SLOT_SOLO;
             t = 0.0f;
         }
-        else
-        {
-            const int s = sc.prim_slot[mobj];
-            int id;
-            const float th = prim_hit<false>(sc.trav, s, make_shear(d), o, d, &id, tmin);
-            t = th >= tmin ? th : 0.0f;
-            slot = th >= tmin ? s : -1;
-        }
+        else slot = enclosing_hit(sc, mobj, o, d, tmin, &t);
     }
     else
     {
@@ -2101,8 +2112,8 @@ static void launch_sdf_extend(const DevScene& sc, const PathState& ps, const int
 {
     if (sc.sdf_trav.node_count > 0) k_sdf_objects<<<grid_s, AR_BLOCK, 0, s>>>(sc, ps, queue, qn);
     if (sc.trav.sdf.count > 0)
-        k_sdf_extend<<<grid_m, AR_BLOCK, 0, s>>>(sc.trav.sdf, sc.sdf_trav.node_count > 0 ? sc.trav.objects : nullptr, ps,
-                                                 queue, qn, &cnt[AR_CNT_SDF]);
+        k_sdf_extend<<<grid_m, AR_BLOCK, 0, s>>>(sc.trav.sdf, sc.sdf_trav.node_count > 0 ? sc.trav.objects : nullptr,
+                                                 sc.trav.object_count, ps, queue, qn, &cnt[AR_CNT_SDF]);
 }
 
 static void launch_sdf_shadow(const DevScene& sc, const PathState& ps, const ShadowQueue& sq, const SdfPending& pend,
