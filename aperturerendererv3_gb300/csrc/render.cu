@@ -599,8 +599,9 @@ __device__ __forceinline__ int sdf_tail_source(bool active, bool exhausted)
 }
 
 // The object a ray is inside of, as the path's media record has it, may be any
-// primitive: a path that starts in one (the camera inside an object) takes the
-// last surface it left.  Rays inside an SDF object test it in the SDF pass.
+// primitive: inside one, a path that scatters off another surface (the camera in a
+// room, the union in glass) takes that one.  Rays inside an SDF object test it in
+// the SDF pass.
 __device__ __forceinline__ bool inside_sdf_object(const Object* objects, int object_count, int id)
 {
     return id >= 0 && id < object_count && objects[id].type == AR_OBJ_SDF;

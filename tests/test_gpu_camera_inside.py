@@ -1,6 +1,6 @@
-"""A camera inside an object: its paths count as inside the last surface they left,
-which may be a mesh triangle or the SDF union as well as an entry of the object
-table.  A mesh renders as the same triangles given one by one as objects, bit for
+"""Paths inside an object (the camera in a room, the SDF union in glass) count as inside
+the last surface they left, which may be a mesh triangle or the SDF union as well
+as an entry of the object table.  A mesh renders as the same triangles given one by one as objects, bit for
 bit, and paths traced to their end in one launch as those traced depth by depth."""
 import numpy as np
 import pytest
@@ -49,8 +49,9 @@ def test_a_mesh_renders_as_its_triangles(cuda_device, room, torus, size, spp):
 @pytest.mark.parametrize("room", list(ROOMS))
 @pytest.mark.parametrize("torus", [False, True])
 @pytest.mark.parametrize("union", [False, True])
-def test_one_launch_and_depth_by_depth_agree(cuda_device, room, torus, union):
+@pytest.mark.parametrize("view", [VIEW, ((0.2, 0.3, 1.7), (-0.05, -0.15, -1.0))])  # from inside, and into the glass
+def test_one_launch_and_depth_by_depth_agree(cuda_device, room, torus, union, view):
     r = _scene(room, True, union, torus)
-    a, b = (r.Render((64, 48), *VIEW, 4, profile=p, **KW) for p in (0, 1))
+    a, b = (r.Render((64, 48), *view, 4, profile=p, **KW) for p in (0, 1))
     assert a.max() > 0 and np.array_equal(a, b)
     assert r.error_word() == 0
